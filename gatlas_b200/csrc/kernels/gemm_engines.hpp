@@ -25,6 +25,12 @@ bool resolve_geometry(const gatlas_matmul_desc *d, Geometry *g);
 int matmul_residual(const Geometry &g, double alpha, double beta, int gemm, const float *A, const float *B,
                     const float *Cin, const float *C, double *out_host, cudaStream_t stream);
 
+// buffer engine's default point for double: FP64 tensor-core instruction
+// (gemm_dmma.cu), for geometries matmul_dmma_takes()
+bool matmul_dmma_takes(const Geometry &g);
+int matmul_dmma(const gatlas_matmul_desc *d, const Geometry &g, const double *A, const double *B, double *C,
+                cudaStream_t stream);
+
 // image engine: SIMT math on TMA tensor-map tile loads (gemm_image.cu)
 int matmul_image_f32(const gatlas_matmul_desc *d, const Geometry &g, const float *A, const float *B,
                      float *C, cudaStream_t stream);
