@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(kThreads2, 1)
     __shared__ volatile int abort_flag;
     __shared__ int mma_aborted;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const uint32_t rank = PAIR ? tc::cluster_ctarank() : 0u;
     const bool leader = rank == 0;
     const int unit = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
@@ -201,25 +201,26 @@ __global__ void __launch_bounds__(kThreads2, 1)
     auto b_tile = [&](int s, int piece) { return smem + s * L::STAGE_BYTES + MD::NP * L::A_TILE + piece * L::B_TILE; };
 
     if (warp == 0) {
-        if (lane == 0) {
-            // ---- TMA producer: one ring position per K slice, across tiles ----
-            const uint32_t full_leader = PAIR ? tc::mapa_shared(smem_u32(&full[0]), 0) : 0u;
-            const uint64_t pol_a = tc::l2_policy_evict_last();
-            int s = 0;
-            uint32_t ph = 0;
-            bool stop = false;
-            for (int64_t t = unit; t < total && !stop; t += units) {
-                int tm, tn, z;
-                decode(t, tm, tn, z);
-                const int m0 = tm * L::TM + (int)rank * 128;
-                const int nb = tn * BN + (int)rank * (PAIR ? 128 : 0);
-                for (int kb = 0; kb < p.kblocks; ++kb) {
-                    if (!wait(&empty[s], ph ^ 1u, kWaitNs)) {
-                        if (!abort_flag) report_fault(p.fault, kFaultTcProducerWait);
-                        abort_flag = 1;
-                        stop = true;
-                        break;
-                    }
+        // ---- TMA producer: one ring position per K slice, across tiles.  As in
+        // the MMA warp below, all lanes walk and wait, one elected lane issues ----
+        const uint32_t full_leader = PAIR ? tc::mapa_shared(smem_u32(&full[0]), 0) : 0u;
+        const uint64_t pol_a = tc::l2_policy_evict_last();
+        int s = 0;
+        uint32_t ph = 0;
+        bool stop = false;
+        for (int64_t t = unit; t < total && !stop; t += units) {
+            int tm, tn, z;
+            decode(t, tm, tn, z);
+            const int m0 = tm * L::TM + (int)rank * 128;
+            const int nb = tn * BN + (int)rank * (PAIR ? 128 : 0);
+            for (int kb = 0; kb < p.kblocks; ++kb) {
+                if (!wait(&empty[s], ph ^ 1u, kWaitNs)) {
+                    if (lane == 0 && !abort_flag) report_fault(p.fault, kFaultTcProducerWait);
+                    abort_flag = 1;
+                    stop = true;
+                    break;
+                }
+                if (tc::elect_one()) {
                     if constexpr (PAIR) {
                         if (leader) mbar_arrive_expect_tx(&full[s], 2 * L::STAGE_BYTES);
                         const uint32_t bar = full_leader + (uint32_t)(s * sizeof(uint64_t));
@@ -236,18 +237,24 @@ __global__ void __launch_bounds__(kThreads2, 1)
                             tma_load_3d(b_tile(s, i), tB[i], kb * BK, nb, z, &full[s]);
                         }
                     }
-                    if (++s == S) {
-                        s = 0;
-                        ph ^= 1u;
-                    }
+                }
+                __syncwarp();
+                if (++s == S) {
+                    s = 0;
+                    ph ^= 1u;
                 }
             }
         }
-        __syncwarp();
     } else if (warp == 1) {
-        if (lane == 0 && leader) {
-            // ---- MMA issuer: segment g (counted across tiles) accumulates into TMEM buffer g & 1 ----
+        if (leader) {
+            // ---- MMA issuer: segment g (counted across tiles) accumulates into
+            // TMEM buffer g & 1.  The whole warp walks the slices, so that
+            // addresses and descriptors stay in uniform registers, and one
+            // elected lane issues: under `lane == 0` each MMA's operands are moved
+            // there first.  Contraction alone, before and after: FP8 8192^3 584 ->
+            // 484 us, BF16 64 x 4096 x 8192 68.6 -> 44.1, split6 8192^3 3927 -> 3889 ----
             constexpr uint32_t idesc = L::IDESC;
+            const uint64_t desc0 = tc::smem_desc_kmajor(smem_u32(smem), L::SBO, L::SWIZZLE);
             const uint32_t empty_self = PAIR ? tc::mapa_shared(smem_u32(&empty[0]), 0) : 0u;
             const uint32_t empty_peer = PAIR ? tc::mapa_shared(smem_u32(&empty[0]), 1) : 0u;
             const uint32_t tfull_self = PAIR ? tc::mapa_shared(smem_u32(&tfull[0]), 0) : 0u;
@@ -258,6 +265,7 @@ __global__ void __launch_bounds__(kThreads2, 1)
             for (int64_t t = unit; t < total && !stop; t += units) {
                 const uint32_t *wb = nullptr;
                 uint32_t wcur = 0, wnext = 0;
+                int in_seg = 0;  // slices of the current segment issued (unscaled modes)
                 if constexpr (MD::SCALED) {
                     int tm, tn, z;
                     decode(t, tm, tn, z);
@@ -276,64 +284,60 @@ __global__ void __launch_bounds__(kThreads2, 1)
                         seg_first = ((wcur >> (kb & 31)) & 1u) != 0;
                         seg_last = k1 == p.kblocks || (((k1 & 31) ? (wcur >> (k1 & 31)) : wnext) & 1u) != 0;
                     } else {
-                        seg_first = (kb % p.seg_kblocks) == 0;
-                        seg_last = (kb % p.seg_kblocks) == p.seg_kblocks - 1 || kb == p.kblocks - 1;
+                        seg_first = in_seg == 0;
+                        seg_last = ++in_seg == p.seg_kblocks || kb == p.kblocks - 1;
+                        if (seg_last) in_seg = 0;
                     }
                     if (seg_first) ++seg;
                     const int b = seg & 1;
-                    if (seg_first) {
-                        // the drain of this buffer's previous segment (both CTAs' for a pair) is done
-                        if (!wait(&tempty[b], ((uint32_t)(seg >> 1) & 1u) ^ 1u, kWaitNs)) {
-                            if (!abort_flag) report_fault(p.fault, kFaultTcMmaWait);
-                            abort_flag = 1;
-                            stop = true;
-                            break;
-                        }
-                        tc::fence_after_sync();
-                    }
-                    if (!wait(&full[s], ph, kWaitNs)) {
-                        if (!abort_flag) report_fault(p.fault, kFaultTcMmaWait);
+                    // the drain of this buffer's previous segment (both CTAs' for a pair) is done
+                    if ((seg_first && !wait(&tempty[b], ((uint32_t)(seg >> 1) & 1u) ^ 1u, kWaitNs)) ||
+                        !wait(&full[s], ph, kWaitNs)) {
+                        if (lane == 0 && !abort_flag) report_fault(p.fault, kFaultTcMmaWait);
                         abort_flag = 1;
                         stop = true;
                         break;
                     }
                     tc::fence_after_sync();
                     const uint32_t d = tmem + (uint32_t)(b * BN);
+                    const uint64_t at = desc0 + (uint64_t)(s * (L::STAGE_BYTES >> 4));
+                    const uint64_t bt = at + ((MD::NP * L::A_TILE) >> 4);
+                    if (tc::elect_one()) {
 #pragma unroll
-                    for (int kk = 0; kk < L::KSTEPS; ++kk) {
+                        for (int kk = 0; kk < L::KSTEPS; ++kk) {
 #pragma unroll
-                        for (int j = 0; j < MD::NPROD; ++j) {
-                            // 32 bytes of K per instruction inside the swizzled rows
-                            const uint32_t a_addr = smem_u32(a_tile(s, MD::pa(j))) + kk * 32;
-                            const uint32_t b_addr = smem_u32(b_tile(s, MD::pb(j))) + kk * 32;
-                            const uint64_t ad = tc::smem_desc_kmajor(a_addr, L::SBO, L::SWIZZLE);
-                            const uint64_t bd = tc::smem_desc_kmajor(b_addr, L::SBO, L::SWIZZLE);
-                            const uint32_t accum = (seg_first && kk == 0 && j == 0) ? 0u : 1u;
-                            if constexpr (MD::SCALED && PAIR) tc::mma_f8_pair(d, ad, bd, idesc, accum);
-                            else if constexpr (MD::SCALED) tc::mma_f8(d, ad, bd, idesc, accum);
-                            else if constexpr (PAIR) tc::mma_bf16_pair(d, ad, bd, idesc, accum);
-                            else tc::mma_bf16(d, ad, bd, idesc, accum);
+                            for (int j = 0; j < MD::NPROD; ++j) {
+                                // 32 bytes of K per instruction inside the swizzled rows
+                                const uint64_t ad = at + ((MD::pa(j) * L::A_TILE + kk * 32) >> 4);
+                                const uint64_t bd = bt + ((MD::pb(j) * L::B_TILE + kk * 32) >> 4);
+                                const uint32_t accum = (seg_first && kk == 0 && j == 0) ? 0u : 1u;
+                                if constexpr (MD::SCALED && PAIR) tc::mma_f8_pair(d, ad, bd, idesc, accum);
+                                else if constexpr (MD::SCALED) tc::mma_f8(d, ad, bd, idesc, accum);
+                                else if constexpr (PAIR) tc::mma_bf16_pair(d, ad, bd, idesc, accum);
+                                else tc::mma_bf16(d, ad, bd, idesc, accum);
+                            }
+                        }
+                        if constexpr (PAIR) {
+                            const uint32_t so = (uint32_t)(s * sizeof(uint64_t)), bo = (uint32_t)(b * sizeof(uint64_t));
+                            tc::commit_pair_to(empty_self + so);
+                            tc::commit_pair_to(empty_peer + so);
+                            if (seg_last) {
+                                tc::commit_pair_to(tfull_self + bo);
+                                tc::commit_pair_to(tfull_peer + bo);
+                            }
+                        } else {
+                            tc::commit_to(&empty[s]);
+                            if (seg_last) tc::commit_to(&tfull[b]);
                         }
                     }
-                    if constexpr (PAIR) {
-                        const uint32_t so = (uint32_t)(s * sizeof(uint64_t)), bo = (uint32_t)(b * sizeof(uint64_t));
-                        tc::commit_pair_to(empty_self + so);
-                        tc::commit_pair_to(empty_peer + so);
-                        if (seg_last) {
-                            tc::commit_pair_to(tfull_self + bo);
-                            tc::commit_pair_to(tfull_peer + bo);
-                        }
-                    } else {
-                        tc::commit_to(&empty[s]);
-                        if (seg_last) tc::commit_to(&tfull[b]);
-                    }
+                    __syncwarp();
                     if (++s == S) {
                         s = 0;
                         ph ^= 1u;
                     }
                 }
             }
-            if (stop) {
+            if (stop && tc::elect_one()) {
                 // every MMA issued before the abort completes before TMEM is freed
                 mma_aborted = 1;
                 if constexpr (PAIR) tc::commit_pair_to(tc::mapa_shared(smem_u32(&mma_done), 0));
@@ -507,7 +511,7 @@ __global__ void __launch_bounds__(kThreads2, 1)
     __shared__ volatile int abort_flag;
     __shared__ int mma_aborted;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int unit = (int)blockIdx.x, units = (int)gridDim.x;
     const int64_t per_batch = (int64_t)p.tiles_m * p.tiles_n;
     const int64_t total = per_batch * p.batch;
@@ -550,79 +554,73 @@ __global__ void __launch_bounds__(kThreads2, 1)
     auto b_tile = [&](int s) { return smem + s * L::STAGE_BYTES + L::A_TILE; };
 
     if (warp == 0) {
-        if (lane == 0) {
-            // ---- TMA producer: one ring position per K slice, across tiles ----
-            int s = 0;
-            uint32_t ph = 0;
-            bool stop = false;
-            for (int64_t t = unit; t < total && !stop; t += units) {
-                int tm, tn, z;
-                decode(t, tm, tn, z);
-                for (int kb = 0; kb < p.kblocks; ++kb) {
-                    if (!tc::wait_timed(&empty[s], ph ^ 1u, kWaitNs, &abort_flag)) {
-                        if (!abort_flag) report_fault(p.fault, kFaultTcProducerWait);
-                        abort_flag = 1;
-                        stop = true;
-                        break;
-                    }
+        // ---- TMA producer: one ring position per K slice, across tiles ----
+        int s = 0;
+        uint32_t ph = 0;
+        bool stop = false;
+        for (int64_t t = unit; t < total && !stop; t += units) {
+            int tm, tn, z;
+            decode(t, tm, tn, z);
+            for (int kb = 0; kb < p.kblocks; ++kb) {
+                if (!tc::wait_timed(&empty[s], ph ^ 1u, kWaitNs, &abort_flag)) {
+                    if (lane == 0 && !abort_flag) report_fault(p.fault, kFaultTcProducerWait);
+                    abort_flag = 1;
+                    stop = true;
+                    break;
+                }
+                if (tc::elect_one()) {
                     mbar_arrive_expect_tx(&full[s], L::STAGE_BYTES);
                     tma_load_3d(a_tile(s), &ta0, kb * BK, tm * L::TM, z, &full[s]);
                     tma_load_3d(b_tile(s), &tb0, kb * BK, tn * BN, z, &full[s]);
-                    if (++s == S) {
-                        s = 0;
-                        ph ^= 1u;
-                    }
+                }
+                __syncwarp();
+                if (++s == S) {
+                    s = 0;
+                    ph ^= 1u;
                 }
             }
         }
-        __syncwarp();
     } else if (warp == 1) {
-        if (lane == 0) {
-            // ---- MMA issuer: each tile accumulates over all of K in TMEM ----
-            constexpr uint32_t idesc = L::IDESC;
-            int s = 0;
-            uint32_t ph = 0, tph = 0;
-            bool stop = false;
-            for (int64_t t = unit; t < total && !stop; t += units, tph ^= 1u) {
-                // the drain has read the previous tile's accumulators
-                if (!tc::wait_timed(&tempty, tph ^ 1u, kWaitNs, &abort_flag)) {
-                    if (!abort_flag) report_fault(p.fault, kFaultTcMmaWait);
+        // ---- MMA issuer: each tile accumulates over all of K in TMEM ----
+        constexpr uint32_t idesc = L::IDESC;
+        const uint64_t desc0 = tc::smem_desc_kmajor(smem_u32(smem), L::SBO, L::SWIZZLE);
+        int s = 0;
+        uint32_t ph = 0, tph = 0;
+        bool stop = false;
+        for (int64_t t = unit; t < total && !stop; t += units, tph ^= 1u) {
+            for (int kb = 0; kb < p.kblocks; ++kb) {
+                // the drain has read the previous tile's accumulators, the slice has landed
+                if ((kb == 0 && !tc::wait_timed(&tempty, tph ^ 1u, kWaitNs, &abort_flag)) ||
+                    !tc::wait_timed(&full[s], ph, kWaitNs, &abort_flag)) {
+                    if (lane == 0 && !abort_flag) report_fault(p.fault, kFaultTcMmaWait);
                     abort_flag = 1;
                     stop = true;
                     break;
                 }
                 tc::fence_after_sync();
-                for (int kb = 0; kb < p.kblocks; ++kb) {
-                    if (!tc::wait_timed(&full[s], ph, kWaitNs, &abort_flag)) {
-                        if (!abort_flag) report_fault(p.fault, kFaultTcMmaWait);
-                        abort_flag = 1;
-                        stop = true;
-                        break;
-                    }
-                    tc::fence_after_sync();
+                const uint64_t at = desc0 + (uint64_t)(s * (L::STAGE_BYTES >> 4)), bt = at + (L::A_TILE >> 4);
+                if (tc::elect_one()) {
 #pragma unroll
                     for (int kk = 0; kk < L::KSTEPS; ++kk) {
-                        const uint32_t a_addr = smem_u32(a_tile(s)) + kk * 32;
-                        const uint32_t b_addr = smem_u32(b_tile(s)) + kk * 32;
-                        const uint64_t bd = tc::smem_desc_kmajor(b_addr, L::SBO, L::SWIZZLE);
                         const uint32_t accum = (kb == 0 && kk == 0) ? 0u : 1u;
-                        tc::mma_bf16(tmem, tc::smem_desc_kmajor(a_addr, L::SBO, L::SWIZZLE), bd, idesc, accum);
-                        tc::mma_bf16(tmem + (uint32_t)BN, tc::smem_desc_kmajor(a_addr + L::A_HALF, L::SBO, L::SWIZZLE),
-                                     bd, idesc, accum);
+                        tc::mma_bf16(tmem, at + (kk * 32 >> 4), bt + (kk * 32 >> 4), idesc, accum);
+                        tc::mma_bf16(tmem + (uint32_t)BN, at + ((L::A_HALF + kk * 32) >> 4), bt + (kk * 32 >> 4), idesc,
+                                     accum);
                     }
                     tc::commit_to(&empty[s]);
-                    if (++s == S) {
-                        s = 0;
-                        ph ^= 1u;
-                    }
+                    if (kb == p.kblocks - 1) tc::commit_to(&tfull);
                 }
-                if (!stop) tc::commit_to(&tfull);
+                __syncwarp();
+                if (++s == S) {
+                    s = 0;
+                    ph ^= 1u;
+                }
             }
-            if (stop) {
-                // every MMA issued before the abort completes before TMEM is freed
-                mma_aborted = 1;
-                tc::commit_to(&mma_done);
-            }
+        }
+        if (stop && tc::elect_one()) {
+            // every MMA issued before the abort completes before TMEM is freed
+            mma_aborted = 1;
+            tc::commit_to(&mma_done);
         }
         __syncwarp();
     } else {

@@ -318,7 +318,7 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_kernel(Params p) {
     __shared__ volatile int abort_flag;
     __shared__ int ring_issued, ring_consumed, mma_aborted;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const uint32_t rank = PAIR ? tc::cluster_ctarank() : 0u;
     const bool leader = rank == 0;
     const int unit = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
@@ -363,40 +363,46 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_kernel(Params p) {
     auto b_tile = [&](int s, int piece) { return smem + s * L::STAGE_BYTES + MD::NP * L::A_TILE + piece * L::B_TILE; };
 
     if (warp == 0) {
-        if (lane == 0) {
-            // ---- producer: one bulk copy per piece tile ----
-            int ring = 0;
-            bool stop = false;
-            TileRec cur;
-            if (t_begin < t_end) cur = p.tiles[t_begin];
-            for (int t = t_begin; t < t_end && !stop; ++t) {
-                // the next record loads while this tile's copies are issued
-                const TileRec next = p.tiles[t + 1 < t_end ? t + 1 : t];
-                // a slice of the B tile is bn rows, and a pair CTA copies its half of
-                // them; rank 1's A tile is the next row block, or (in a tile of 128
-                // rows or fewer) rank 0's again, whose products are never stored
-                const uint32_t b_slice = (uint32_t)cur.bn * kRowBytes;
-                const uint32_t b_bytes = PAIR ? b_slice / 2 : b_slice;
-                const int64_t a_off = (PAIR && rank == 1 && cur.rows > BM) ? (int64_t)cur.kt * kATileBytes : 0;
-                const int64_t b_off = PAIR ? (int64_t)rank * b_bytes : 0;
-                for (int kb = 0; kb < cur.kt; ++kb, ++ring) {
-                    const int s = ring % S;
-                    if (!wait(&empty[s], ((uint32_t)(ring / S) & 1u) ^ 1u, kWaitNs)) {
-                        if (!abort_flag) report_fault(p.fault, kFaultTcProducerWait);
-                        abort_flag = 1;
-                        stop = true;
-                        break;
-                    }
+        // ---- producer: one bulk copy per piece tile (all lanes walk and wait,
+        // one elected lane issues, as in the MMA warp) ----
+        int ring = 0, s = 0;
+        uint32_t ph = 0;
+        bool stop = false;
+        TileRec cur;
+        if (t_begin < t_end) cur = p.tiles[t_begin];
+        for (int t = t_begin; t < t_end && !stop; ++t) {
+            // the next record loads while this tile's copies are issued
+            const TileRec next = p.tiles[t + 1 < t_end ? t + 1 : t];
+            // a slice of the B tile is bn rows, and a pair CTA copies its half of
+            // them; rank 1's A tile is the next row block, or (in a tile of 128
+            // rows or fewer) rank 0's again, whose products are never stored
+            const uint32_t b_slice = (uint32_t)cur.bn * kRowBytes;
+            const uint32_t b_bytes = PAIR ? b_slice / 2 : b_slice;
+            const int64_t a_off = (PAIR && rank == 1 && cur.rows > BM) ? (int64_t)cur.kt * kATileBytes : 0;
+            const int64_t b_off = PAIR ? (int64_t)rank * b_bytes : 0;
+            for (int kb = 0; kb < cur.kt; ++kb, ++ring) {
+                if (!wait(&empty[s], ph ^ 1u, kWaitNs)) {
+                    if (lane == 0 && !abort_flag) report_fault(p.fault, kFaultTcProducerWait);
+                    abort_flag = 1;
+                    stop = true;
+                    break;
+                }
+                if (tc::elect_one()) {
                     mbar_arrive_expect_tx(&full[s], MD::NP * (kATileBytes + b_bytes));
                     for (int i = 0; i < MD::NP; ++i) {
                         bulk_g2s(a_tile(s, i), cur.a[i] + a_off + (int64_t)kb * kATileBytes, kATileBytes, &full[s]);
                         bulk_g2s(b_tile(s, i), cur.b[i] + b_off + (int64_t)kb * b_slice, b_bytes, &full[s]);
                     }
                 }
-                cur = next;
+                __syncwarp();
+                if (++s == S) {
+                    s = 0;
+                    ph ^= 1u;
+                }
             }
-            ring_issued = ring;
+            cur = next;
         }
+        if (lane == 0) ring_issued = ring;
         __syncwarp();
     } else if (warp == 1) {
         if (PAIR && !leader && lane == 0) {
@@ -417,74 +423,81 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_kernel(Params p) {
                     tc::mbar_arrive_remote(full_leader + (uint32_t)(s * sizeof(uint64_t)));
                 }
             }
-        } else if (lane == 0) {
-            // ---- MMA issuer ----
+        } else if (!PAIR || leader) {
+            // ---- MMA issuer: the whole warp walks the slices, so that addresses
+            // and descriptors stay in uniform registers, and one elected lane
+            // issues: under `lane == 0` each MMA's operands are moved there
+            // first, which takes longer than an MMA of width 64 or 128 ----
+            const uint64_t desc0 = tc::smem_desc_kmajor(smem_u32(smem), L::SBO, L::SWIZZLE);
             const uint32_t empty_self = PAIR ? tc::mapa_shared(smem_u32(&empty[0]), 0) : 0u;
             const uint32_t empty_peer = PAIR ? tc::mapa_shared(smem_u32(&empty[0]), 1) : 0u;
             const uint32_t tfull_self = PAIR ? tc::mapa_shared(smem_u32(&tfull[0]), 0) : 0u;
             const uint32_t tfull_peer = PAIR ? tc::mapa_shared(smem_u32(&tfull[0]), 1) : 0u;
-            int ring = 0, seg = 0;
+            int ring = 0, seg = 0, s = 0;
+            uint32_t ph = 0;
             bool stop = false;
             int2 cur = make_int2(0, 0);  // (kt, bn)
             if (t_begin < t_end) cur = make_int2(p.tiles[t_begin].kt, p.tiles[t_begin].bn);
             for (int t = t_begin; t < t_end && !stop; ++t) {
                 const int tn = t + 1 < t_end ? t + 1 : t;
                 const int2 next = make_int2(p.tiles[tn].kt, p.tiles[tn].bn);
-                const int kt = cur.x;
-                const uint32_t idesc = tc::idesc_bf16_f32(PAIR ? 2 * BM : BM, cur.y);
+                const int kt = __shfl_sync(0xffffffffu, cur.x, 0);
+                const uint32_t idesc = tc::idesc_bf16_f32(PAIR ? 2 * BM : BM, __shfl_sync(0xffffffffu, cur.y, 0));
                 cur = next;
+                int in_seg = 0;  // slices of the current segment issued
                 for (int kb = 0; kb < kt; ++kb, ++ring) {
                     const int b = seg & 1;
-                    const bool seg_first = (kb % p.seg_kblocks) == 0;
-                    const bool seg_last = (kb % p.seg_kblocks) == p.seg_kblocks - 1 || kb == kt - 1;
-                    if (seg_first) {
-                        if (!wait(&tempty[b], ((uint32_t)(seg >> 1) & 1u) ^ 1u, kWaitNs)) {
-                            if (!abort_flag) report_fault(p.fault, kFaultTcMmaWait);
-                            abort_flag = 1;
-                            stop = true;
-                            break;
-                        }
-                        tc::fence_after_sync();
-                    }
-                    const int s = ring % S;
-                    if (!wait(&full[s], (uint32_t)(ring / S) & 1u, kWaitNs)) {
-                        if (!abort_flag) report_fault(p.fault, kFaultTcMmaWait);
+                    const bool seg_first = in_seg == 0;
+                    const bool seg_last = ++in_seg == p.seg_kblocks || kb == kt - 1;
+                    if ((seg_first && !wait(&tempty[b], ((uint32_t)(seg >> 1) & 1u) ^ 1u, kWaitNs)) ||
+                        !wait(&full[s], ph, kWaitNs)) {
+                        if (lane == 0 && !abort_flag) report_fault(p.fault, kFaultTcMmaWait);
                         abort_flag = 1;
                         stop = true;
                         break;
                     }
                     tc::fence_after_sync();
                     const uint32_t d = tmem + (uint32_t)(b * 256);
+                    const uint64_t at = desc0 + (uint64_t)(s * (L::STAGE_BYTES >> 4));
+                    const uint64_t bt = at + ((MD::NP * L::A_TILE) >> 4);
+                    if (tc::elect_one()) {
 #pragma unroll
-                    for (int kk = 0; kk < L::KSTEPS; ++kk) {
+                        for (int kk = 0; kk < L::KSTEPS; ++kk) {
 #pragma unroll
-                        for (int j = 0; j < MD::NPROD; ++j) {
-                            const uint32_t a_addr = smem_u32(a_tile(s, MD::pa(j))) + kk * 32;
-                            const uint32_t b_addr = smem_u32(b_tile(s, MD::pb(j))) + kk * 32;
-                            const uint64_t ad = tc::smem_desc_kmajor(a_addr, L::SBO, L::SWIZZLE);
-                            const uint64_t bd = tc::smem_desc_kmajor(b_addr, L::SBO, L::SWIZZLE);
-                            const uint32_t accum = (seg_first && kk == 0 && j == 0) ? 0u : 1u;
-                            if constexpr (PAIR) tc::mma_bf16_pair(d, ad, bd, idesc, accum);
-                            else tc::mma_bf16(d, ad, bd, idesc, accum);
+                            for (int j = 0; j < MD::NPROD; ++j) {
+                                const uint64_t ad = at + ((MD::pa(j) * L::A_TILE + kk * 32) >> 4);
+                                const uint64_t bd = bt + ((MD::pb(j) * L::B_TILE + kk * 32) >> 4);
+                                const uint32_t accum = (seg_first && kk == 0 && j == 0) ? 0u : 1u;
+                                if constexpr (PAIR) tc::mma_bf16_pair(d, ad, bd, idesc, accum);
+                                else tc::mma_bf16(d, ad, bd, idesc, accum);
+                            }
+                        }
+                        if constexpr (PAIR) {
+                            const uint32_t so = (uint32_t)(s * sizeof(uint64_t)), bo = (uint32_t)(b * sizeof(uint64_t));
+                            tc::commit_pair_to(empty_self + so);
+                            tc::commit_pair_to(empty_peer + so);
+                            if (seg_last) {
+                                tc::commit_pair_to(tfull_self + bo);
+                                tc::commit_pair_to(tfull_peer + bo);
+                            }
+                        } else {
+                            tc::commit_to(&empty[s]);
+                            if (seg_last) tc::commit_to(&tfull[b]);
                         }
                     }
-                    if constexpr (PAIR) {
-                        const uint32_t so = (uint32_t)(s * sizeof(uint64_t)), bo = (uint32_t)(b * sizeof(uint64_t));
-                        tc::commit_pair_to(empty_self + so);
-                        tc::commit_pair_to(empty_peer + so);
-                        if (seg_last) {
-                            tc::commit_pair_to(tfull_self + bo);
-                            tc::commit_pair_to(tfull_peer + bo);
-                        }
-                    } else {
-                        tc::commit_to(&empty[s]);
-                        if (seg_last) tc::commit_to(&tfull[b]);
+                    __syncwarp();
+                    if (seg_last) {
+                        ++seg;
+                        in_seg = 0;
                     }
-                    if (seg_last) ++seg;
+                    if (++s == S) {
+                        s = 0;
+                        ph ^= 1u;
+                    }
                 }
             }
-            ring_consumed = ring;
-            if (stop) {
+            if (lane == 0) ring_consumed = ring;
+            if (stop && tc::elect_one()) {
                 // every MMA issued before the abort completes before TMEM is freed
                 mma_aborted = 1;
                 if constexpr (PAIR) tc::commit_pair_to(tc::mapa_shared(smem_u32(&mma_done), 0));
