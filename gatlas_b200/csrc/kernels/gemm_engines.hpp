@@ -58,6 +58,11 @@ int matmul_tc(const gatlas_matmul_desc *d, const Geometry &g, const float *A, co
 int tc_supported(const gatlas_matmul_desc *d);
 size_t tc_workspace_bytes(const gatlas_matmul_desc *d, const Geometry &g);
 namespace tcg {
+// one-launch contraction of products of few tiles (gemm_tc_direct.cu): its
+// tile width for a product, 0 where the two-pass path serves it
+int direct_width(const gatlas_matmul_desc *d, const Geometry &g, const float *A, const float *B, const float *C);
+int matmul_direct(const gatlas_matmul_desc *d, const Geometry &g, int bn, const float *A, const float *B, float *C,
+                  cudaStream_t stream);
 // host-buffer pipeline of the tensor-core engines (gemm_tc.cu)
 bool host_pipeline_ok(const gatlas_matmul_desc *d, const Geometry &g);
 size_t host_pipeline_bytes(const gatlas_matmul_desc *d, const Geometry &g);

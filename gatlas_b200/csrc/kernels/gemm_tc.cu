@@ -1597,6 +1597,10 @@ int matmul_tc(const gatlas_matmul_desc *d, const Geometry &g, const float *A, co
         return gatlas_matmul_f32(&s, A, B, C, nullptr, 0, stream);
     }
     if (!ws) {
+        // one launch without prepared operands where that is faster (a caller's
+        // workspace holds them afterwards, and a selected tiling is kept)
+        const int bn = g_tc_pair == 1 ? direct_width(d, g, A, B, C) : 0;
+        if (bn) return matmul_direct(d, g, bn, A, B, C, stream);
         ws = device_scratch(pl.total);
         if (!ws) return set_error(GATLAS_ERR_NOMEM, "matmul: scratch of %zu bytes", pl.total);
         ws_bytes = pl.total;

@@ -175,7 +175,9 @@ int gatlas_matmul_f64(const gatlas_matmul_desc *d, const double *A, const double
  * writes the BF16 pieces of A and B into the workspace
  * (gatlas_matmul_workspace_size bytes, 1024-byte aligned); run contracts the
  * prepared pieces into C and may be repeated.  gatlas_matmul_f32 with a TC_*
- * engine is prepare followed by run.  No reference counterpart (the reference
+ * engine is prepare followed by run; without a workspace, products of few
+ * tiles run in one launch that splits the operands on the way to the tensor
+ * cores (BF16 and split engines, "tc_pair" 1), with identical results.  No reference counterpart (the reference
  * regenerates and re-uploads operands per run, KernelMatmulBuffer.hpp:83-171). */
 int gatlas_matmul_tc_prepare(const gatlas_matmul_desc *d, const float *A, const float *B, void *workspace,
                              size_t workspace_bytes, void *stream);
