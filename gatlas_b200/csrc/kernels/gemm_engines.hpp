@@ -31,6 +31,11 @@ bool matmul_dmma_takes(const Geometry &g);
 int matmul_dmma(const gatlas_matmul_desc *d, const Geometry &g, const double *A, const double *B, double *C,
                 cudaStream_t stream);
 
+// ... and for float: FP32 SIMT math on asynchronous copies (gemm_ffma.cu)
+bool matmul_ffma_takes(const Geometry &g);
+int matmul_ffma(const gatlas_matmul_desc *d, const Geometry &g, const float *A, const float *B, float *C,
+                cudaStream_t stream);
+
 // image engine: SIMT math on TMA tensor-map tile loads (gemm_image.cu)
 int matmul_image_f32(const gatlas_matmul_desc *d, const Geometry &g, const float *A, const float *B,
                      float *C, cudaStream_t stream);
