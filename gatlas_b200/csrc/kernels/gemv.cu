@@ -7,23 +7,31 @@
 // row-major A.
 //
 // B200 design (both layouts read every byte of A exactly once, 16-byte loads):
-//  * trans_a == 0 (row-major): for long rows (at least 4 x 256 vectors) a CTA
+//  * trans_a == 0 (row-major): for long rows (at least 4 x 256 loads) a CTA
 //    owns two rows at a time and its 256 threads stride across them in
-//    16-byte vectors, reduced in a fixed order (warp butterfly, then the 8
+//    16-byte vectors (single elements where rows are off the 16-byte grid),
+//    reduced in a fixed order (warp butterfly, then the 8
 //    warps in shared memory); otherwise a warp owns ROWS rows at a time, its
 //    lanes striding across the row with UNROLL loads per row in flight and a
 //    fixed butterfly shuffle reduction.  x is read through the L1-cached
 //    read-only path.
-//  * trans_a == 1 (column-major): a CTA owns 32*VW adjacent columns (one
+//  * trans_a == 1 (column-major): one launch of clusters whose CTAs own the row
+//    segments of a column block and add their sums over distributed shared
+//    memory (gemv_cols.cuh) where the matrix has enough columns; otherwise a
+//    CTA owns 32*VW adjacent columns (one
 //    16-byte vector per lane) and one segment of the rows; its 8 warps take
 //    interleaved rows, partial sums are combined across warps in a fixed order
 //    in shared memory, and across the S row segments by the last CTA of each
 //    column block (partials in a workspace, arrival counter per column block).
 // Results are deterministic: the order depends only on (M, N) and the SM count.
+// Measured (device time, before and after): 3001 x 7013 column-major 23.8 ->
+// 17.2 us, row-major 45.6 -> 17.6; 1024 x 32767 207 -> 32; 1024^2 column-major
+// 12.5 -> 4.3, row-major 4.5 -> 3.3; 32768 x 1024 column-major 36.5 -> 22.1.
 #include <algorithm>
 
 #include "../common.cuh"
 #include "../device_state.cuh"
+#include "gemv_cols.cuh"
 
 namespace gatlas {
 
@@ -73,7 +81,32 @@ constexpr int kGemvWarps = kGemvThreads / 32;
 // ---------------------------------------------------------------------------
 // row-major A
 // ---------------------------------------------------------------------------
-template <typename T, int VW, int ROWS, int UNROLL>
+// The last, partial group of a thread's strided vectors: all loads at once, as
+// in a whole group, with vectors past the row read as its last one and left
+// out of the sums (loading them one by one cost a memory latency each: rows of
+// 32767 floats ran 207 us where rows of 32768 ran 26).
+template <typename T, typename V, int ROWS, int UNROLL, int STRIDE>
+__device__ __forceinline__ void row_tail(T (&acc)[ROWS], const V *const (&arow)[ROWS], const V *x, size_t c, size_t nvec) {
+    V av[ROWS][UNROLL], xv[UNROLL];
+#pragma unroll
+    for (int u = 0; u < UNROLL; ++u) {
+        const size_t i = min(c + (size_t)u * STRIDE, nvec - 1);
+        xv[u] = __ldg(x + i);
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) av[r][u] = __ldcs(arow[r] + i);
+    }
+#pragma unroll
+    for (int u = 0; u < UNROLL; ++u) {
+        const bool in = c + (size_t)u * STRIDE < nvec;
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) acc[r] = in ? dot_acc(acc[r], av[r][u], xv[u]) : acc[r];
+    }
+}
+
+// FEW: few warps per SM, so the tail of a row loads at once (row_tail); with
+// many the plain remainder loop is shorter and its latencies overlap (32768 x
+// 1023: 29 us, 33 with row_tail; 1024^2 the other way round).
+template <typename T, int VW, int ROWS, int UNROLL, bool FEW>
 __global__ void __launch_bounds__(kGemvThreads)
     gemv_rows_kernel(GemvArgs a) {
     using V = typename VecT<T, VW>::type;
@@ -112,10 +145,14 @@ __global__ void __launch_bounds__(kGemvThreads)
 #pragma unroll
                 for (int r = 0; r < ROWS; ++r) acc[r] = dot_acc(acc[r], av[r][u], xv[u]);
         }
-        for (; c < nvec; c += 32) {
-            const V xv = __ldg(x + c);
+        if constexpr (FEW) {
+            if (c < nvec) row_tail<T, V, ROWS, UNROLL, 32>(acc, arow, x, c, nvec);
+        } else {
+            for (; c < nvec; c += 32) {
+                const V xv = __ldg(x + c);
 #pragma unroll
-            for (int r = 0; r < ROWS; ++r) acc[r] = dot_acc(acc[r], __ldcs(arow[r] + c), xv);
+                for (int r = 0; r < ROWS; ++r) acc[r] = dot_acc(acc[r], __ldcs(arow[r] + c), xv);
+            }
         }
 #pragma unroll
         for (int r = 0; r < ROWS; ++r) {
@@ -176,11 +213,7 @@ __global__ void __launch_bounds__(kGemvThreads)
 #pragma unroll
                 for (int r = 0; r < RB; ++r) acc[r] = dot_acc(acc[r], av[r][u], xv[u]);
         }
-        for (; c < nvec; c += kGemvThreads) {
-            const V xv = __ldg(x + c);
-#pragma unroll
-            for (int r = 0; r < RB; ++r) acc[r] = dot_acc(acc[r], __ldcs(arow[r] + c), xv);
-        }
+        if (c < nvec) row_tail<T, V, RB, UNROLL, kGemvThreads>(acc, arow, x, c, nvec);
 #pragma unroll
         for (int r = 0; r < RB; ++r) {
 #pragma unroll
@@ -359,6 +392,71 @@ static bool gemv_vec_ok(const gatlas_matvec_desc *d, const T *A, const T *x) {
     return ok;
 }
 
+// Column-major products whose segments fit one cluster (gemv_cols.cuh).
+// nseg == 0: the general kernel, with partial sums in a workspace, serves it:
+// too few column blocks for clusters of 8 to fill the GPU, or doubles off the
+// 16-byte grid (26 us at 2479 x 5702 against 33).
+struct ClusterPlan {
+    int variant, nseg;
+    size_t width;
+};
+
+template <typename T>
+static ClusterPlan cluster_plan(const gatlas_matvec_desc *d, bool vec_ok) {
+    ClusterPlan c{0, 0, 0};
+    const size_t batch = d->batch ? d->batch : 1;
+    if (d->n == 0 || (sizeof(T) == 8 && !vec_ok)) return c;
+    // narrow blocks with more rows in flight up to 4096 columns (2048 off the
+    // 16-byte grid), wide ones beyond: 3000 x 7012 18.7 us (W = 32) and 28.7
+    // (W = 128), 16384^2 167 and 161, 1024 x 32768 24.7 and 107
+    const bool narrow = d->m <= (vec_ok ? 4096u : 2048u);
+    c.variant = narrow ? 0 : 1;
+    c.width = narrow ? 32 : (vec_ok ? 32 * (16 / sizeof(T)) : 64);
+    const size_t blocks = (d->m + c.width - 1) / c.width * batch;
+    if (blocks * 8 < (size_t)sm_count() || blocks / batch > 0x7fffffffu) return c;
+    // at most 640 CTAs, in clusters of 1, 2, 4 or 8, of at least 64 rows each
+    int nseg = 8;
+    while (nseg > 1 && (blocks * (size_t)nseg > 640 || (size_t)nseg * 64 > d->n)) nseg /= 2;
+    c.nseg = nseg;
+    return c;
+}
+
+template <typename T>
+static int launch_cluster(const GemvArgs &g, const ClusterPlan &cp, bool vec_ok, size_t batch, cudaStream_t stream) {
+    gvc::Args a;
+    a.A = g.A, a.x = g.x, a.y = g.y;
+    a.M = g.M, a.N = g.N, a.lda = g.lda;
+    a.stride_a = g.stride_a, a.stride_x = g.stride_x, a.stride_y = g.stride_y;
+    a.alpha = g.alpha, a.beta = g.beta, a.gemv = g.gemv;
+    a.seg_len = (g.N + cp.nseg - 1) / cp.nseg;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((g.M + cp.width - 1) / cp.width), (unsigned)cp.nseg, (unsigned)batch);
+    cfg.blockDim = dim3(gvc::kThreads, 1, 1);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1;
+    attr[0].val.clusterDim.y = (unsigned)cp.nseg;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    constexpr int V = 16 / (int)sizeof(T);
+    cudaError_t e;
+    if constexpr (sizeof(T) == 4) {
+        if (vec_ok)
+            e = cp.variant == 0 ? cudaLaunchKernelEx(&cfg, gvc::gemv_cols_cluster_kernel<T, true, 8, V, 16>, a)
+                                : cudaLaunchKernelEx(&cfg, gvc::gemv_cols_cluster_kernel<T, true, 32, V, 8>, a);
+        else
+            e = cp.variant == 0 ? cudaLaunchKernelEx(&cfg, gvc::gemv_cols_cluster_kernel<T, false, 16, 2, 16>, a)
+                                : cudaLaunchKernelEx(&cfg, gvc::gemv_cols_cluster_kernel<T, false, 16, 4, 8>, a);
+    } else {
+        e = cp.variant == 0 ? cudaLaunchKernelEx(&cfg, gvc::gemv_cols_cluster_kernel<T, true, 16, V, 8>, a)
+                            : cudaLaunchKernelEx(&cfg, gvc::gemv_cols_cluster_kernel<T, true, 32, V, 8>, a);
+    }
+    if (e != cudaSuccess) return set_error(GATLAS_ERR_CUDA, "gemv_cols_cluster_kernel: %s", cudaGetErrorString(e));
+    return check_launch("gemv_cols_cluster_kernel");
+}
+
 template <typename T>
 static size_t matvec_ws(const gatlas_matvec_desc *d, const void *A, const void *x) {
     if (!d || !d->trans_a) return 0;
@@ -399,28 +497,36 @@ static int matvec_launch(const gatlas_matvec_desc *d, const T *A, const T *x, T 
     const bool vec_ok = gemv_vec_ok<T>(d, A, x);
     const int sms = sm_count();
     if (!d->trans_a) {
-        constexpr int UNROLL = 4;
         constexpr int VWV = 16 / sizeof(T);
-        if (vec_ok && d->n / VWV >= (size_t)UNROLL * kGemvThreads) {
-            // long rows: a CTA per RB rows (see gemv_rowblock_kernel)
+        const size_t per_row = vec_ok ? d->n / VWV : d->n;  // loads per row
+        if (per_row >= (size_t)4 * kGemvThreads) {
+            // long rows: a CTA per RB rows (see gemv_rowblock_kernel); elements
+            // of rows off the 16-byte grid are a quarter (half) as wide, so twice
+            // as many are in flight where the row holds that many
             constexpr int RB = 2;
             const size_t nblocks = (d->m + RB - 1) / RB;
             const size_t cap = (size_t)sms * 64 / (batch < 8 ? batch : 8);
             dim3 g((unsigned)(nblocks < cap ? nblocks : cap), (unsigned)batch);
-            gemv_rowblock_kernel<T, VWV, RB, UNROLL><<<g, kGemvThreads, 0, stream>>>(a);
+            if (vec_ok) gemv_rowblock_kernel<T, VWV, RB, 4><<<g, kGemvThreads, 0, stream>>>(a);
+            else if (per_row >= (size_t)8 * kGemvThreads) gemv_rowblock_kernel<T, 1, RB, 8><<<g, kGemvThreads, 0, stream>>>(a);
+            else gemv_rowblock_kernel<T, 1, RB, 4><<<g, kGemvThreads, 0, stream>>>(a);
             return check_launch("gemv_rowblock_kernel");
         }
-        constexpr int ROWS = 2;
-        const size_t warps_needed = (d->m + ROWS - 1) / ROWS;
+        // shorter rows: a warp per two rows, or per row (and twice the loads of
+        // it in flight) while that leaves SMs with few warps
+        const bool few = d->m * batch < (size_t)sms * 4 * kGemvWarps;
+        const int rows = few ? 1 : 2;
+        const size_t warps_needed = (d->m + rows - 1) / rows;
         size_t grid = (warps_needed + kGemvWarps - 1) / kGemvWarps;
         const size_t cap = (size_t)sms * 8 / (batch < 8 ? batch : 8);
         if (grid > cap) grid = cap ? cap : 1;
         dim3 g((unsigned)grid, (unsigned)batch);
         if (vec_ok) {
-            constexpr int VW = 16 / sizeof(T);
-            gemv_rows_kernel<T, VW, ROWS, 4><<<g, kGemvThreads, 0, stream>>>(a);
+            if (few) gemv_rows_kernel<T, VWV, 1, 8, true><<<g, kGemvThreads, 0, stream>>>(a);
+            else gemv_rows_kernel<T, VWV, 2, 4, false><<<g, kGemvThreads, 0, stream>>>(a);
         } else {
-            gemv_rows_kernel<T, 1, ROWS, 4><<<g, kGemvThreads, 0, stream>>>(a);
+            if (few) gemv_rows_kernel<T, 1, 1, 16, true><<<g, kGemvThreads, 0, stream>>>(a);
+            else gemv_rows_kernel<T, 1, 2, 4, false><<<g, kGemvThreads, 0, stream>>>(a);
         }
         return check_launch("gemv_rows_kernel");
     }
@@ -430,13 +536,16 @@ static int matvec_launch(const gatlas_matvec_desc *d, const T *A, const T *x, T 
     unsigned *counters = nullptr;
     if (pl.nseg > 1) {
         const size_t need = pl.part_bytes + pl.counter_bytes;
+        if (ws && ws_bytes < need)
+            return set_error(GATLAS_ERR_INVALID, "matvec: workspace %zu < %zu bytes", ws_bytes, need);
+        if (ws && !aligned_to(ws, 256)) return set_error(GATLAS_ERR_INVALID, "matvec: workspace must be 256-byte aligned");
+    }
+    if (const ClusterPlan cp = cluster_plan<T>(d, vec_ok); cp.nseg) return launch_cluster<T>(a, cp, vec_ok, batch, stream);
+    if (pl.nseg > 1) {
+        const size_t need = pl.part_bytes + pl.counter_bytes;
         if (!ws) {
             ws = device_scratch(need);
             if (!ws) return set_error(GATLAS_ERR_NOMEM, "matvec: scratch of %zu bytes", need);
-        } else if (ws_bytes < need) {
-            return set_error(GATLAS_ERR_INVALID, "matvec: workspace %zu < %zu bytes", ws_bytes, need);
-        } else if (!aligned_to(ws, 256)) {
-            return set_error(GATLAS_ERR_INVALID, "matvec: workspace must be 256-byte aligned");
         }
         partial = static_cast<T *>(ws);
         counters = reinterpret_cast<unsigned *>(static_cast<char *>(ws) + pl.part_bytes);
