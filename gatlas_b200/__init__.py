@@ -171,13 +171,29 @@ def _torch():
 
 
 def _ptr(t):
-    return None if t is None else ctypes.c_void_p(t.data_ptr())
+    return None if t is None else t.data_ptr()
+
+
+_current_raw_stream = None
 
 
 def _stream(stream=None):
-    torch = _torch()
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return ctypes.c_void_p(s.cuda_stream)
+    """The stream's handle; by default the current device's current stream.
+    Asked of torch's C layer where it has the query (0.2 us a call; building a
+    Stream object takes 3.3 us, a third of a small call)."""
+    if stream is not None:
+        return stream.cuda_stream
+    global _current_raw_stream
+    if _current_raw_stream is None:
+        torch = _torch()
+        torch.cuda.current_stream()  # initialises CUDA
+        raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+        device = getattr(torch._C, "_cuda_getDevice", None)
+        if raw is not None and device is not None:
+            _current_raw_stream = lambda: raw(device())  # noqa: E731
+        else:
+            _current_raw_stream = lambda: torch.cuda.current_stream().cuda_stream  # noqa: E731
+    return _current_raw_stream()
 
 
 def _engine(engine) -> int:
@@ -215,9 +231,8 @@ def saxpy(alpha, x, y, out=None, engine="buffer", stream=None):
 
 def matvec_desc(M, N, trans_a=False, gemv=False, alpha=1.0, beta=0.0, engine="buffer",
                 lda=0, batch=1, stride_a=0, stride_x=0, stride_y=0) -> MatvecDesc:
-    return MatvecDesc(engine=_engine(engine), gemv=int(bool(gemv)), trans_a=int(bool(trans_a)),
-                      reserved0=0, m=M, n=N, lda=lda, batch=batch, stride_a=stride_a,
-                      stride_x=stride_x, stride_y=stride_y, alpha=alpha, beta=beta)
+    return MatvecDesc(_engine(engine), 1 if gemv else 0, 1 if trans_a else 0, 0, M, N, lda, batch, stride_a,
+                      stride_x, stride_y, alpha, beta)
 
 
 def matvec(A, x, M, N, y=None, trans_a=False, gemv=False, alpha=1.0, beta=0.0,
@@ -226,8 +241,8 @@ def matvec(A, x, M, N, y=None, trans_a=False, gemv=False, alpha=1.0, beta=0.0,
     row-major; trans_a=True → column-major (N rows of M)."""
     torch = _torch()
     _require_cuda(A, x, y)
-    if y is None:
-        y = torch.zeros(batch * M, dtype=A.dtype, device=A.device)
+    if y is None:  # read only where beta is used
+        y = (torch.zeros if gemv else torch.empty)(batch * M, dtype=A.dtype, device=A.device)
     d = matvec_desc(M, N, trans_a, gemv, alpha, beta, engine, batch=batch)
     fn = lib().gatlas_matvec_f32 if A.dtype == torch.float32 else lib().gatlas_matvec_f64
     ws = _ptr(workspace)
@@ -246,11 +261,8 @@ def matmul_desc(M, N, K, trans_a=False, trans_b=False, gemm=False, alpha=1.0, be
                 stride_a=0, stride_b=0, stride_c=0) -> MatmulDesc:
     t = tuple(tile or ())
     gh, gw, bh, bw, vl, x = t + (0,) * (6 - len(t))
-    return MatmulDesc(engine=_engine(engine), gemm=int(bool(gemm)), trans_a=int(bool(trans_a)),
-                      trans_b=int(bool(trans_b)), m=M, n=N, k=K, lda=lda, ldb=ldb, ldc=ldc,
-                      batch=batch, stride_a=stride_a, stride_b=stride_b, stride_c=stride_c,
-                      alpha=alpha, beta=beta, group_h=gh, group_w=gw, block_h=bh, block_w=bw,
-                      vector_length=vl, extra=x)
+    return MatmulDesc(_engine(engine), 1 if gemm else 0, 1 if trans_a else 0, 1 if trans_b else 0, M, N, K,
+                      lda, ldb, ldc, batch, stride_a, stride_b, stride_c, alpha, beta, gh, gw, bh, bw, vl, x)
 
 
 def matmul(A, B, M, N, K, C=None, trans_a=False, trans_b=False, gemm=False, alpha=1.0,
