@@ -835,7 +835,7 @@ __global__ void __launch_bounds__(256) split_transpose_kernel(SplitArgs a) {
 // ---------------------------------------------------------------------------
 constexpr int kQBlock = 128;
 
-struct QuantArgs {
+struct QuantOperand {
     const float *src;
     int64_t rows, K, Kp, ld, src_stride;
     int transposed;   // element (r,k) at src[k*ld + r] instead of src[r*ld + k]
@@ -843,6 +843,13 @@ struct QuantArgs {
     uint8_t *codes;   // [batch][rows][Kp]
     float *scales;    // [batch][rblocks][kblocks]
     int64_t rblocks, kblocks;
+};
+
+// One launch quantises one operand or both: CTAs [0, split) the first
+// operand's blocks, the others the second's.
+struct QuantArgs {
+    QuantOperand op[2];
+    int64_t split;
 };
 
 // Staged code words: row r (0..127) holds 32 words of 4 codes; word w is
@@ -856,23 +863,31 @@ __device__ __forceinline__ int qt_index(int r, int w) { return r * 32 + (w ^ ((r
 // same real number, hence identical; elsewhere (s subnormal or huge) divide.
 __device__ __forceinline__ float scale_down(float x, float s, float r) { return r != 0.0f ? x * r : __fdiv_rn(x, s); }
 
+// Four codes; one conversion instruction makes two.
 __device__ __forceinline__ uint32_t e4m3_pack4(float s, float r, float x0, float x1, float x2, float x3) {
     if (s == 0.0f) return 0u;
-    const uint32_t b0 = __nv_cvt_float_to_fp8(scale_down(x0, s, r), __NV_SATFINITE, __NV_E4M3);
-    const uint32_t b1 = __nv_cvt_float_to_fp8(scale_down(x1, s, r), __NV_SATFINITE, __NV_E4M3);
-    const uint32_t b2 = __nv_cvt_float_to_fp8(scale_down(x2, s, r), __NV_SATFINITE, __NV_E4M3);
-    const uint32_t b3 = __nv_cvt_float_to_fp8(scale_down(x3, s, r), __NV_SATFINITE, __NV_E4M3);
-    return b0 | (b1 << 8) | (b2 << 16) | (b3 << 24);
+    const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(scale_down(x0, s, r), scale_down(x1, s, r)), __NV_SATFINITE,
+                                                 __NV_E4M3);
+    const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(scale_down(x2, s, r), scale_down(x3, s, r)), __NV_SATFINITE,
+                                                 __NV_E4M3);
+    return lo | (hi << 16);
 }
 
-constexpr int kQThreads = 512;  // 32 values per thread; two CTAs (1024 threads) per SM
+// 32 values per thread; three CTAs per SM (40 registers), so that loads are in
+// flight while others reduce and convert: both operands of 8192^3 in 145 us
+// (158 with two CTAs; 158 as two launches with one-value conversions before)
+constexpr int kQThreads = 512;
 
-__global__ void __launch_bounds__(kQThreads, 2) quant_fp8_kernel(QuantArgs a) {
+__global__ void __launch_bounds__(kQThreads, 3) quant_fp8_kernel(const __grid_constant__ QuantArgs args) {
     constexpr int G = kQBlock * kQBlock / 4 / kQThreads;  // groups of 4 values per thread
     __shared__ uint32_t qt[kQBlock * 32];
     __shared__ float red[kQThreads / 32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int64_t r0 = (int64_t)blockIdx.y * kQBlock, k0 = (int64_t)blockIdx.x * kQBlock, z = blockIdx.z;
+    const bool second = blockIdx.x >= args.split;
+    const QuantOperand &a = args.op[second ? 1 : 0];
+    const int64_t block = (int64_t)blockIdx.x - (second ? args.split : 0);
+    const int64_t rb = block / a.kblocks, kb = block - rb * a.kblocks;
+    const int64_t r0 = rb * kQBlock, k0 = kb * kQBlock, z = blockIdx.y;
     const float *src = a.src + z * a.src_stride;
     // 4*G values per thread as G groups of 4 consecutive elements of the
     // stored inner dimension (k for direct sources, rows for transposed ones)
@@ -926,7 +941,7 @@ __global__ void __launch_bounds__(kQThreads, 2) quant_fp8_kernel(QuantArgs a) {
         s = ldexpf(1.0f, j);
         if (isfinite(amax) && j >= -126 && j <= 126) rcp = ldexpf(1.0f, -j);  // 1/s, exact and normal
     }
-    if (tid == 0) a.scales[(z * a.rblocks + blockIdx.y) * a.kblocks + blockIdx.x] = s;
+    if (tid == 0) a.scales[(z * a.rblocks + rb) * a.kblocks + kb] = s;
     if (!a.transposed) {
 #pragma unroll
         for (int i = 0; i < G; ++i) {
@@ -1013,9 +1028,9 @@ static bool make_plan(const gatlas_matmul_desc *d, const Geometry &g, Plan *pl) 
     return true;
 }
 
-static int launch_quant(bool transposed, const float *src, int64_t rows, int64_t K, int64_t Kp, int64_t ld,
-                        int64_t src_stride, int64_t batch, uint8_t *codes, float *scales, cudaStream_t stream) {
-    QuantArgs a;
+static QuantOperand quant_operand(bool transposed, const float *src, int64_t rows, int64_t K, int64_t Kp, int64_t ld,
+                                  int64_t src_stride, int64_t batch, uint8_t *codes, float *scales) {
+    QuantOperand a;
     a.src = src;
     a.rows = rows;
     a.K = K;
@@ -1028,8 +1043,18 @@ static int launch_quant(bool transposed, const float *src, int64_t rows, int64_t
     a.scales = scales;
     a.rblocks = (rows + kQBlock - 1) / kQBlock;
     a.kblocks = (K + kQBlock - 1) / kQBlock;
-    if (a.rblocks > 65535) return set_error(GATLAS_ERR_INVALID, "matmul: too many rows for the FP8 pass");
-    dim3 gr((unsigned)a.kblocks, (unsigned)a.rblocks, (unsigned)batch);
+    return a;
+}
+
+// Quantises `first` and, when not null, `second` in one launch.
+static int launch_quant(const QuantOperand &first, const QuantOperand *second, int64_t batch, cudaStream_t stream) {
+    QuantArgs a;
+    a.op[0] = first;
+    a.op[1] = second ? *second : first;
+    a.split = first.rblocks * first.kblocks;
+    if (first.rblocks > 65535 || (second && second->rblocks > 65535))
+        return set_error(GATLAS_ERR_INVALID, "matmul: too many rows for the FP8 pass");
+    dim3 gr((unsigned)(a.split + (second ? second->rblocks * second->kblocks : 0)), (unsigned)batch);
     quant_fp8_kernel<<<gr, kQThreads, 0, stream>>>(a);
     return check_launch("quant_fp8_kernel");
 }
@@ -1099,8 +1124,9 @@ static WsPtrs ws_ptrs(const Plan &pl, void *ws) {
 // Tiling of C for M > 128 ("tc_pair"): 1 = what measures fastest on B200 --
 // CTA pairs for the split engines (17-19 % fewer cycles per 8192^3 launch
 // than 128 x 256 single CTAs), 256 x 256 single-CTA tiles for one-product
-// BF16 over all of K (35 % fewer), 128 x 256 single CTAs for FP8 (pairs
-// measured 30 % slower); 2 = CTA pairs always; 0 = 128 x 256 always.
+// BF16 over all of K (35 % fewer); FP8 on CTA pairs once every pair of SMs has
+// a tile (8192^3 398 us against 454 on single CTAs, 4096^3 84 and 90, but
+// 2048^3 26.1 and 25.2); 2 = CTA pairs always; 0 = 128 x 256 always.
 static int g_tc_pair = 1;
 // Rows of C per raster group of the persistent kernels (multiple of 128).
 static int g_tc_group_rows = kGroupM * 128;
@@ -1109,63 +1135,74 @@ static int g_tc_group_rows = kGroupM * 128;
 // same speed.
 static int g_tc_l2_hint = 1;
 
-// FP8 segment plan, one thread per tile: a run of at most seg_kblocks
-// 128-deep blocks whose scale products sa * sb are equal for every 128 x 128
-// block of the tile accumulates in TMEM and is promoted, scaled once (exact:
-// the scales are powers of two).  Writes the tile's segment count, its
-// segment-start bits and each segment's scale products.  Single CTAs
-// (pair == 0) have 128 x 256 tiles: one A block, two column halves, products
-// (a b0, a b1) per segment.  CTA pairs (pair == 1) have 256 x 256 tiles: the
-// MMAs of both CTAs share their segments, so a run ends where any of the four
-// products changes; per segment the plan holds (a0 b0, a0 b1) for the
-// leader's rows and (a1 b0, a1 b1) for the peer's.
-__global__ void __launch_bounds__(128)
+// FP8 segment plan, one warp per tile, 32 blocks of K at a time: a run of at
+// most seg_kblocks 128-deep blocks whose scale products sa * sb are equal for
+// every 128 x 128 block of the 256 x 256 block the tile lies in accumulates in
+// TMEM and is promoted, scaled once (exact: the scales are powers of two).
+// Writes the tile's segment count, its segment-start bits and each segment's
+// scale products.  Single CTAs (pair == 0) have 128 x 256 tiles: one A block,
+// two column halves, products (a b0, a b1) per segment.  CTA pairs (pair == 1)
+// have 256 x 256 tiles, whose MMAs share their segments: per segment the plan
+// holds (a0 b0, a0 b1) for the leader's rows and (a1 b0, a1 b1) for the
+// peer's.  Runs end where any of the four products changes in either case, so
+// both tilings promote alike and give identical results.  (One thread per tile
+// walking K serially took 6.6 us of a 4096^3 product.)
+constexpr int kPlanWarps = 4;
+
+__global__ void __launch_bounds__(32 * kPlanWarps)
     fp8_plan_kernel(const float *scale_a, const float *scale_b, int64_t sa_stride, int64_t sb_stride, int tiles_m,
                     int tiles_n, int batch, int kblocks, int nblocks_m, int nblocks_n, int seg_kblocks, int words,
                     int pair, int *nseg, uint32_t *bits, float2 *q) {
-    const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31;
+    const int64_t idx = (int64_t)blockIdx.x * kPlanWarps + (threadIdx.x >> 5);
     if (idx >= (int64_t)tiles_m * tiles_n * batch) return;
     const int tn = (int)(idx % tiles_n);
     const int64_t rest = idx / tiles_n;
     const int tm = (int)(rest % tiles_m);
     const int64_t z = rest / tiles_m;
-    const int ma0 = pair ? 2 * tm : tm, ma1 = 2 * tm + 1;
+    const int ma0 = pair ? 2 * tm : tm & ~1, ma1 = ma0 + 1;
     const float *sa0 = scale_a + z * sa_stride + (int64_t)ma0 * kblocks;
-    const float *sa1 = pair && ma1 < nblocks_m ? scale_a + z * sa_stride + (int64_t)ma1 * kblocks : nullptr;
+    const float *sa1 = ma1 < nblocks_m ? scale_a + z * sa_stride + (int64_t)ma1 * kblocks : nullptr;
     const int nb0 = 2 * tn, nb1 = 2 * tn + 1;
     const float *sb0 = nb0 < nblocks_n ? scale_b + z * sb_stride + (int64_t)nb0 * kblocks : nullptr;
     const float *sb1 = nb1 < nblocks_n ? scale_b + z * sb_stride + (int64_t)nb1 * kblocks : nullptr;
     uint32_t *wb = bits + idx * words;
     float2 *qt = q + idx * kblocks * (pair ? 2 : 1);
-    int s = -1, run = 0;
-    float prev[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    uint32_t w = 0;
-    for (int kb = 0; kb < kblocks; ++kb) {
-        const float a0 = sa0[kb], a1 = sa1 ? sa1[kb] : 0.0f;
-        const float b0 = sb0 ? sb0[kb] : 0.0f, b1 = sb1 ? sb1[kb] : 0.0f;
+    int count = 0, run0 = 0;                       // segments so far; first block of the run of equal products
+    float carry[4] = {0.0f, 0.0f, 0.0f, 0.0f};     // the products of the block before this word
+    for (int w = 0; w < words; ++w) {
+        const int kb = w * 32 + lane;
+        const bool in = kb < kblocks;
+        const float a0 = in ? sa0[kb] : 0.0f, a1 = in && sa1 ? sa1[kb] : 0.0f;
+        const float b0 = in && sb0 ? sb0[kb] : 0.0f, b1 = in && sb1 ? sb1[kb] : 0.0f;
         const float cur[4] = {sb0 ? __fmul_rn(a0, b0) : 0.0f, sb1 ? __fmul_rn(a0, b1) : 0.0f,
                               sa1 && sb0 ? __fmul_rn(a1, b0) : 0.0f, sa1 && sb1 ? __fmul_rn(a1, b1) : 0.0f};
-        bool start = kb == 0 || run == seg_kblocks;
-        for (int i = 0; i < 4; ++i) start = start || cur[i] != prev[i];
+        bool change = kb == 0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float up = __shfl_up_sync(0xffffffffu, cur[i], 1);
+            change = change || cur[i] != (lane ? up : carry[i]);
+            carry[i] = __shfl_sync(0xffffffffu, cur[i], 31);
+        }
+        const uint32_t changes = __ballot_sync(0xffffffffu, change && in);
+        const uint32_t upto = changes & (0xffffffffu >> (31 - lane));  // changes at or before this block
+        const int first = upto ? w * 32 + 31 - __clz(upto) : run0;
+        const bool start = in && (kb - first) % seg_kblocks == 0;
+        const uint32_t starts = __ballot_sync(0xffffffffu, start);
         if (start) {
-            ++s;
-            run = 0;
+            const int s = count + __popc(starts & ((1u << lane) - 1u));
             if (pair) {
                 qt[2 * s] = make_float2(cur[0], cur[1]);
                 qt[2 * s + 1] = make_float2(cur[2], cur[3]);
             } else {
-                qt[s] = make_float2(cur[0], cur[1]);
+                qt[s] = tm & 1 ? make_float2(cur[2], cur[3]) : make_float2(cur[0], cur[1]);
             }
-            w |= 1u << (kb & 31);
         }
-        ++run;
-        for (int i = 0; i < 4; ++i) prev[i] = cur[i];
-        if ((kb & 31) == 31 || kb == kblocks - 1) {
-            wb[kb >> 5] = w;
-            w = 0;
-        }
+        if (lane == 0) wb[w] = starts;
+        count += __popc(starts);
+        if (changes) run0 = w * 32 + 31 - __clz(changes);
     }
-    nseg[idx] = s + 1;
+    if (lane == 0) nseg[idx] = count;
 }
 
 // Encodes the tensor map of C for the TMA-store epilogue (32 x 32 boxes,
@@ -1273,7 +1310,9 @@ template <int MODE>
 static int launch_tc(const Geometry &g, const Plan &pl, const WsPtrs &w, float *C, double alpha, double beta,
                      int gemm, int seg_kblocks, cudaStream_t stream) {
     using L = Layout<MODE>;
-    const bool pair = g.M > BM && (g_tc_pair == 2 || (g_tc_pair == 1 && (MODE == 1 || MODE == 2)));
+    const int64_t pair_tiles = ((g.M + 2 * BM - 1) / (2 * BM)) * ((g.N + BN - 1) / BN) * g.batch;
+    const bool pair = g.M > BM && (g_tc_pair == 2 || (g_tc_pair == 1 && (MODE == 1 || MODE == 2 ||
+                                                                         (MODE == 3 && pair_tiles >= sm_count() / 2))));
     CUtensorMap ta[3], tb[3];
     const uint64_t row_bytes = (uint64_t)pl.Kp * pl.elem;
     const uint64_t adims[3] = {(uint64_t)pl.Kp, (uint64_t)g.M, (uint64_t)g.batch};
@@ -1330,7 +1369,7 @@ static int launch_tc(const Geometry &g, const Plan &pl, const WsPtrs &w, float *
         const int64_t tiles = tiles_m * tiles_n * g.batch;
         if (tiles > 0) {
             const int words = (int)((p.kblocks + 31) / 32);
-            fp8_plan_kernel<<<(unsigned)((tiles + 127) / 128), 128, 0, stream>>>(
+            fp8_plan_kernel<<<(unsigned)((tiles + kPlanWarps - 1) / kPlanWarps), 32 * kPlanWarps, 0, stream>>>(
                 w.sa, w.sb, p.scale_a_stride, p.scale_b_stride, (int)tiles_m, (int)tiles_n, (int)g.batch,
                 p.kblocks, p.nblocks_m, p.nblocks_n, p.seg_kblocks, words, pair ? 1 : 0, w.plan_nseg, w.plan_bits,
                 w.plan_q);
@@ -1362,11 +1401,11 @@ int tc_prepare(const gatlas_matmul_desc *d, const Geometry &g, const float *A, c
     const WsPtrs w = ws_ptrs(pl, ws);
     // A is K-major already when not transposed; B is K-major when transposed.
     if (pl.mode == 3) {
-        rc = launch_quant(g.ta, A, g.M, g.K, pl.Kp, g.lda, g.stride_a, g.batch, static_cast<uint8_t *>(w.a[0]), w.sa,
-                          stream);
-        if (rc) return rc;
-        return launch_quant(!g.tb, B, g.N, g.K, pl.Kp, g.ldb, g.stride_b, g.batch, static_cast<uint8_t *>(w.b[0]),
-                            w.sb, stream);
+        const QuantOperand b = quant_operand(!g.tb, B, g.N, g.K, pl.Kp, g.ldb, g.stride_b, g.batch,
+                                             static_cast<uint8_t *>(w.b[0]), w.sb);
+        return launch_quant(quant_operand(g.ta, A, g.M, g.K, pl.Kp, g.lda, g.stride_a, g.batch,
+                                          static_cast<uint8_t *>(w.a[0]), w.sa),
+                            &b, g.batch, stream);
     }
     __nv_bfloat16 *ap[3], *bp[3];
     for (int i = 0; i < 3; ++i) {
@@ -1410,8 +1449,10 @@ static int prepare_a_rows(const Plan &pl, const Geometry &g, const float *A, int
     const float *src = g.ta ? A + r0 : A + r0 * g.lda;  // stored K x M: a column block
     const int64_t rows = r1 - r0;
     if (pl.mode == 3)
-        return launch_quant(g.ta, src, rows, g.K, pl.Kp, g.lda, 0, 1, static_cast<uint8_t *>(w.a[0]) + r0 * pl.Kp,
-                            w.sa + (r0 / kQBlock) * pl.kblocks, s);
+        return launch_quant(quant_operand(g.ta, src, rows, g.K, pl.Kp, g.lda, 0, 1,
+                                          static_cast<uint8_t *>(w.a[0]) + r0 * pl.Kp,
+                                          w.sa + (r0 / kQBlock) * pl.kblocks),
+                            nullptr, 1, s);
     __nv_bfloat16 *ap[3];
     for (int i = 0; i < 3; ++i)
         ap[i] = w.a[i] ? static_cast<__nv_bfloat16 *>(w.a[i]) + r0 * pl.Kp : nullptr;
@@ -1420,7 +1461,8 @@ static int prepare_a_rows(const Plan &pl, const Geometry &g, const float *A, int
 
 static int prepare_b(const Plan &pl, const Geometry &g, const float *B, const WsPtrs &w, cudaStream_t s) {
     if (pl.mode == 3)
-        return launch_quant(!g.tb, B, g.N, g.K, pl.Kp, g.ldb, 0, 1, static_cast<uint8_t *>(w.b[0]), w.sb, s);
+        return launch_quant(quant_operand(!g.tb, B, g.N, g.K, pl.Kp, g.ldb, 0, 1, static_cast<uint8_t *>(w.b[0]), w.sb),
+                            nullptr, 1, s);
     __nv_bfloat16 *bp[3];
     for (int i = 0; i < 3; ++i) bp[i] = static_cast<__nv_bfloat16 *>(w.b[i]);
     return launch_split(pl.np, !g.tb, B, g.N, g.K, pl.Kp, g.ldb, 0, 1, bp, s);

@@ -148,8 +148,8 @@ int gatlas_matvec_f32_noalloc(const gatlas_matvec_desc *d, const float *A, const
  * tc_prepare workspace holds [A codes][B codes][A scales][B scales][plan],
  * codes K-major [batch][rows][Kp] (Kp = K rounded up to 16), scales
  * [batch][rows/128][K/128], each part 1024-byte aligned; tc_run writes the
- * plan (each 128 x 256 tile's runs of equally scaled blocks) before it
- * contracts. */
+ * plan (each tile's runs of blocks over which the 256 x 256 block of C it lies
+ * in is equally scaled) before it contracts. */
 typedef struct gatlas_matmul_desc {
     int32_t engine;
     int32_t gemm;
@@ -202,7 +202,8 @@ int gatlas_matmul_f32_host(const gatlas_matmul_desc *d, const float *A, const fl
  * tile C.  1 (default): CTA pairs (cta_group::2, a 256 x 256 tile per pair,
  * each CTA staging half of B) for split3 and split6; 256 x 256 tiles on
  * single CTAs for one-product BF16 over all of K once there are at least as
- * many such tiles as SMs; one CTA per 128 x 256 tile otherwise.  2: CTA
+ * many such tiles as SMs; CTA pairs for FP8 once there are as many 256 x 256
+ * tiles as SM pairs; one CTA per 128 x 256 tile otherwise.  2: CTA
  * pairs always.  0: 128 x 256 tiles always.  Results are bit-identical in
  * every case (same pieces, same MMA order, same promotion).
  * "tc_group_rows": rows of C per raster group of the persistent
