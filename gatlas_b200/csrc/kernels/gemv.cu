@@ -213,7 +213,15 @@ __global__ void __launch_bounds__(kGemvThreads)
 #pragma unroll
                 for (int r = 0; r < RB; ++r) acc[r] = dot_acc(acc[r], av[r][u], xv[u]);
         }
-        if (c < nvec) row_tail<T, V, RB, UNROLL, kGemvThreads>(acc, arow, x, c, nvec);
+        if constexpr (VW == 1) {
+            if (c < nvec) row_tail<T, V, RB, UNROLL, kGemvThreads>(acc, arow, x, c, nvec);
+        } else {  // (row_tail would cost the fifth CTA per SM its registers: 16 -> 21 us at 1272 x 16108)
+            for (; c < nvec; c += kGemvThreads) {
+                const V xv = __ldg(x + c);
+#pragma unroll
+                for (int r = 0; r < RB; ++r) acc[r] = dot_acc(acc[r], __ldcs(arow[r] + c), xv);
+            }
+        }
 #pragma unroll
         for (int r = 0; r < RB; ++r) {
 #pragma unroll
@@ -406,17 +414,20 @@ static ClusterPlan cluster_plan(const gatlas_matvec_desc *d, bool vec_ok) {
     ClusterPlan c{0, 0, 0};
     const size_t batch = d->batch ? d->batch : 1;
     if (d->n == 0 || (sizeof(T) == 8 && !vec_ok)) return c;
-    // narrow blocks with more rows in flight up to 4096 columns (2048 off the
-    // 16-byte grid), wide ones beyond: 3000 x 7012 18.7 us (W = 32) and 28.7
-    // (W = 128), 16384^2 167 and 161, 1024 x 32768 24.7 and 107
-    const bool narrow = d->m <= (vec_ok ? 4096u : 2048u);
+    // narrow blocks with more rows in flight, as long as clusters of them fit the
+    // GPU at once; wide ones beyond (float: 5296 x 14956 49.7 us narrow and 60.5
+    // wide, 16384^2 167 and 156), 4096 doubles, 2048 off the 16-byte grid
+    const bool narrow = d->m <= (!vec_ok ? 2048u : sizeof(T) == 8 ? 4096u : 96u * (unsigned)sm_count());
     c.variant = narrow ? 0 : 1;
     c.width = narrow ? 32 : (vec_ok ? 32 * (16 / sizeof(T)) : 64);
     const size_t blocks = (d->m + c.width - 1) / c.width * batch;
     if (blocks * 8 < (size_t)sm_count() || blocks / batch > 0x7fffffffu) return c;
-    // at most 640 CTAs, in clusters of 1, 2, 4 or 8, of at least 64 rows each
+    // clusters of up to 8 CTAs, as many in all as are resident for certain: four
+    // CTAs per SM, three of the float kernels with 16 rows in flight (5596 x
+    // 19076 doubles 196 us with 704 CTAs, 135 with 528), each of 64 rows at least
+    const size_t resident = (size_t)sm_count() * (sizeof(T) == 4 && narrow ? 3 : 4);
     int nseg = 8;
-    while (nseg > 1 && (blocks * (size_t)nseg > 640 || (size_t)nseg * 64 > d->n)) nseg /= 2;
+    while (nseg > 1 && (blocks * (size_t)nseg > resident || (size_t)nseg * 64 > d->n)) --nseg;
     c.nseg = nseg;
     return c;
 }

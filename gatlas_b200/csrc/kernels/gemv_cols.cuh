@@ -43,6 +43,22 @@ __device__ __forceinline__ double ld_peer(uint32_t addr, double) {
     return v;
 }
 
+// Streaming loads that stay where they are written: left to itself the
+// compiler pairs loads with their multiply-adds to save registers, and half as
+// many are in flight.
+__device__ __forceinline__ void load_vec(const float *p, float (&v)[4]) {
+    asm volatile("ld.global.cs.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "l"(p));
+}
+__device__ __forceinline__ void load_vec(const double *p, double (&v)[2]) {
+    asm volatile("ld.global.cs.v2.f64 {%0, %1}, [%2];" : "=d"(v[0]), "=d"(v[1]) : "l"(p));
+}
+__device__ __forceinline__ void load_one(const float *p, float &v) {
+    asm volatile("ld.global.cs.f32 %0, [%1];" : "=f"(v) : "l"(p));
+}
+__device__ __forceinline__ void load_one(const double *p, double &v) {
+    asm volatile("ld.global.cs.f64 %0, [%1];" : "=d"(v) : "l"(p));
+}
+
 // T; VEC: 16-byte loads (CPL = 16 / sizeof(T)); LPR lanes per row; U row groups in flight
 template <typename T, bool VEC, int LPR, int CPL, int U>
 __global__ void __launch_bounds__(kThreads) gemv_cols_cluster_kernel(Args a) {
@@ -70,13 +86,10 @@ __global__ void __launch_bounds__(kThreads) gemv_cols_cluster_kernel(Args a) {
     constexpr int STEP = kWarps * RPW;  // rows per group of all warps
     size_t j = j0 + (size_t)w * RPW + lr;
     auto load = [&](const T *row, T (&v)[CPL]) {
-        if constexpr (VEC) {
-            const uint4 q = __ldcs(reinterpret_cast<const uint4 *>(row + off[0]));
-            memcpy(v, &q, 16);
-        } else {
+        if constexpr (VEC) load_vec(row + off[0], v);
+        else
 #pragma unroll
-            for (int c = 0; c < CPL; ++c) v[c] = __ldcs(row + off[c]);
-        }
+            for (int c = 0; c < CPL; ++c) load_one(row + off[c], v[c]);
     };
     const T *row = A + j * a.lda;
     const size_t adv = (size_t)STEP * a.lda;
