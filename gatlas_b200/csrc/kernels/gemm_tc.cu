@@ -88,7 +88,52 @@ struct Params {
 // quarter (w % 4) and column half (w - 2) / 4.
 constexpr int kDrainWarps = 8;
 constexpr int kThreads2 = 32 * (2 + kDrainWarps);
+// The persistent kernel's roles are whole warpgroups: warps 0 and 1 as above (2
+// and 3 idle), the drain warps 4..11.  The first group gives its registers to
+// the drain, whose 128 sums a thread do not fit the 168 that 384 threads start
+// with: 128 x 40 + 256 x 232 = 384 x 168.
+constexpr int kThreadsP = 384;
+constexpr int kIssueRegs = 40, kDrainRegs = 232;
+static_assert(128 * kIssueRegs + 256 * kDrainRegs <= kThreadsP * 168, "register split");
 constexpr uint32_t kTmemCols2 = 2 * BN;  // two accumulator buffers
+
+// Plain-store epilogue of one warp's 32 x 32 chunk (beta != 0, or rows of C off
+// the 16-byte grid, where a TMA store cannot go): v holds row `lane`'s 32
+// columns; the chunk passes through the warp's staging tile (16-byte chunk j of
+// row r at j ^ (r & 7)), so that C is read and written a row at a time, lanes
+// across the columns.  One row per lane instead touched 32 rows per
+// instruction: 300 x 5298 x 161 BF16 took 32 us, now 17; 7049 x 2166 x 828
+// 120, now 51.
+template <typename F>
+__device__ __forceinline__ void store_chunk_plain(uint8_t *stage, int lane, const Params &p, float *C, int64_t row0,
+                                                  int64_t col0, F value) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+        *reinterpret_cast<float4 *>(stage + lane * 128 + ((j ^ (lane & 7)) << 4)) =
+            make_float4(value(4 * j), value(4 * j + 1), value(4 * j + 2), value(4 * j + 3));
+    __syncwarp();
+    const int64_t col = col0 + lane;
+    const int rows = (int)(p.M - row0 < 32 ? p.M - row0 : 32);
+    const bool read = p.gemm && p.beta != 0.0f;
+    if (col < p.N) {
+        float *c = C + row0 * p.ldc + col;
+#pragma unroll
+        for (int r0 = 0; r0 < 32; r0 += 8) {
+            float old[8];
+#pragma unroll
+            for (int r = 0; r < 8; ++r) old[r] = read && r0 + r < rows ? c[(r0 + r) * p.ldc] : 0.0f;
+#pragma unroll
+            for (int r = 0; r < 8; ++r) {
+                const int rr = r0 + r;
+                if (rr >= rows) continue;
+                const float a = *reinterpret_cast<const float *>(stage + rr * 128 + (((lane >> 2) ^ (rr & 7)) << 4) +
+                                                                 (lane & 3) * 4);
+                c[rr * p.ldc] = p.gemm ? __fmaf_rn(p.alpha, a, p.beta == 0.0f ? 0.0f : p.beta * old[r]) : a;
+            }
+        }
+    }
+    __syncwarp();  // the staging tile is read
+}
 
 // ---------------------------------------------------------------------------
 // Persistent contraction: one CTA (or CTA pair) per SM walks
@@ -120,7 +165,7 @@ constexpr uint32_t kTmemCols2 = 2 * BN;  // two accumulator buffers
 // MMAs or copies can still touch its shared memory.
 // ---------------------------------------------------------------------------
 template <int MODE, bool PAIR>
-__global__ void __launch_bounds__(kThreads2, 1)
+__global__ void __launch_bounds__(kThreadsP, 1)
     tc_gemm_persistent_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CUtensorMap ta1,
                               const __grid_constant__ CUtensorMap ta2, const __grid_constant__ CUtensorMap tb0,
                               const __grid_constant__ CUtensorMap tb1, const __grid_constant__ CUtensorMap tb2,
@@ -200,6 +245,7 @@ __global__ void __launch_bounds__(kThreads2, 1)
     auto a_tile = [&](int s, int piece) { return smem + s * L::STAGE_BYTES + piece * L::A_TILE; };
     auto b_tile = [&](int s, int piece) { return smem + s * L::STAGE_BYTES + MD::NP * L::A_TILE + piece * L::B_TILE; };
 
+    if (warp < 4) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kIssueRegs));
     if (warp == 0) {
         // ---- TMA producer: one ring position per K slice, across tiles.  As in
         // the MMA warp below, all lanes walk and wait, one elected lane issues ----
@@ -345,14 +391,14 @@ __global__ void __launch_bounds__(kThreads2, 1)
             }
         }
         __syncwarp();
-    } else {
+    } else if (warp >= 4) {
         // ---- drain: promote each segment into round-to-nearest FP32 sums; then C ----
-        const int quarter = warp & 3, half = (warp - 2) >> 2;
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kDrainRegs));
+        const int quarter = warp & 3, half = (warp - 4) >> 2;
         const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
         const uint32_t tempty_leader = PAIR ? tc::mapa_shared(smem_u32(&tempty[0]), 0) : 0u;
-        uint8_t *stage = smem + L::EPI_OFFSET + (warp - 2) * kEpiTileBytes;
+        uint8_t *stage = smem + L::EPI_OFFSET + (warp - 4) * kEpiTileBytes;
         const int nseg = (p.kblocks + p.seg_kblocks - 1) / p.seg_kblocks;
-        const bool vec_ok = (p.ldc % 4 == 0) && ((reinterpret_cast<uintptr_t>(p.C) & 15) == 0) && (p.stride_c % 4 == 0);
         int seg = -1;
         bool ok = true;
         for (int64_t t = unit; t < total && ok; t += units) {
@@ -386,7 +432,7 @@ __global__ void __launch_bounds__(kThreads2, 1)
                     break;
                 }
                 tc::fence_after_sync();
-                // 16-column loads keep the drain within the 168-register cap
+                // 16 columns at a time: wider loads hold more registers for nothing
 #pragma unroll
                 for (int c = 0; c < BN / 2 / 16; ++c) {
                     uint32_t r[16];
@@ -436,32 +482,12 @@ __global__ void __launch_bounds__(kThreads2, 1)
                         bulk_commit();
                     }
                 }
-            } else {
-                const int64_t row = row0 + lane;
-                float *crow = p.C + (int64_t)z * p.stride_c + row * p.ldc;
-                if (row < p.M) {
+            } else if (row0 < p.M) {
 #pragma unroll
-                    for (int j = 0; j < BN / 2; j += 4) {
-                        float v[4];
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            const int64_t col = col0 + j + e;
-                            if (p.gemm) {
-                                const float bc = (p.beta == 0.0f || col >= p.N) ? 0.0f : p.beta * crow[col];
-                                v[e] = __fmaf_rn(p.alpha, acc[j + e], bc);
-                            } else {
-                                v[e] = acc[j + e];
-                            }
-                        }
-                        if (vec_ok && col0 + j + 3 < p.N) {
-                            *reinterpret_cast<float4 *>(crow + col0 + j) = make_float4(v[0], v[1], v[2], v[3]);
-                        } else {
-#pragma unroll
-                            for (int e = 0; e < 4; ++e)
-                                if (col0 + j + e < p.N) crow[col0 + j + e] = v[e];
-                        }
-                    }
-                }
+                for (int c = 0; c < BN / 2 / 32; ++c)
+                    if (col0 + c * 32 < p.N)
+                        store_chunk_plain(stage, lane, p, p.C + (int64_t)z * p.stride_c, row0, col0 + c * 32,
+                                          [&](int e) { return acc[c * 32 + e]; });
             }
         }
         if (lane == 0) bulk_wait<0>();  // this warp's C stores are complete
@@ -630,7 +656,6 @@ __global__ void __launch_bounds__(kThreads2, 1)
         const int quarter = warp & 3, half = (warp - 2) >> 2;
         const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
         uint8_t *stage = smem + L::EPI_OFFSET + (warp - 2) * kEpiTileBytes;
-        const bool vec_ok = (p.ldc % 4 == 0) && ((reinterpret_cast<uintptr_t>(p.C) & 15) == 0) && (p.stride_c % 4 == 0);
         uint32_t tph = 0;
         for (int64_t t = unit; t < total; t += units, tph ^= 1u) {
             int tm, tn, z;
@@ -681,33 +706,9 @@ __global__ void __launch_bounds__(kThreads2, 1)
                         tma_store_3d(&tcout, stage, (int32_t)col0, (int32_t)row0, z);
                         bulk_commit();
                     }
-                } else {
-                    const int64_t row = row0 + lane;
-                    if (row < p.M) {
-                        float *crow = p.C + (int64_t)z * p.stride_c + row * p.ldc;
-#pragma unroll
-                        for (int j = 0; j < 32; j += 4) {
-                            float v[4];
-#pragma unroll
-                            for (int e = 0; e < 4; ++e) {
-                                const int64_t col = col0 + j + e;
-                                const float a = __uint_as_float(r[j + e]);
-                                if (p.gemm) {
-                                    const float bc = (p.beta == 0.0f || col >= p.N) ? 0.0f : p.beta * crow[col];
-                                    v[e] = __fmaf_rn(p.alpha, a, bc);
-                                } else {
-                                    v[e] = a;
-                                }
-                            }
-                            if (vec_ok && col0 + j + 3 < p.N) {
-                                *reinterpret_cast<float4 *>(crow + col0 + j) = make_float4(v[0], v[1], v[2], v[3]);
-                            } else {
-#pragma unroll
-                                for (int e = 0; e < 4; ++e)
-                                    if (col0 + j + e < p.N) crow[col0 + j + e] = v[e];
-                            }
-                        }
-                    }
+                } else if (row0 < p.M && col0 < p.N) {
+                    store_chunk_plain(stage, lane, p, p.C + (int64_t)z * p.stride_c, row0, col0,
+                                      [&](int e) { return __uint_as_float(r[e]); });
                 }
             }
         }
@@ -1243,7 +1244,7 @@ static int launch_persistent(const CUtensorMap *ta, const CUtensorMap *tb, const
     CUtensorMap tcout = ta[0];  // unused unless tma_store
     c_tensor_map(g, p, &tcout);
     cudaLaunchConfig_t cfg = {};
-    cfg.blockDim = dim3(kThreads2, 1, 1);
+    cfg.blockDim = dim3(kThreadsP, 1, 1);
     cfg.dynamicSmemBytes = (size_t)smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];

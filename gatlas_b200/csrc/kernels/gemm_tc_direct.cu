@@ -535,16 +535,17 @@ Source source(const float *p, int64_t ld, int64_t rows, int64_t stride, int64_t 
 // Tile width of the one-launch contraction for a product, 0 where the
 // two-pass path serves it: whichever of the two is estimated faster.
 //
-// Microseconds per 64 k of one tile, and per launch, from a sweep of 29 shapes
+// Microseconds per 64 k of one tile, and per launch, from a sweep of 36 shapes
 // (device time, B200).  A 64-row tile of width 32, a 128-row tile of width 32
-// and of width 64 take 0.40 / 0.60 / 0.80 (BF16), 0.52 / 0.75 / 1.05 (split3)
-// and 0.75 / 1.00 / 1.40 (split6), over half more where an operand has to be
-// read in pairs; the two-pass contraction 0.30 / 0.85 / 1.85 on its wider
-// tiles, after a split pass at 4 TB/s and two more launches.  Either side of
-// the line, direct against two-pass: 64 x 4096 x 8192 BF16 56 and 86 us,
-// split3 69 and 197, split6 100 and 350; 1024^3 split3 21 and 27;
-// 512^3 BF16 9.5 and 12.8; 1536^3 split3 53 and 37; 128 x 128 x 4096 BF16 40
-// and 28; 2000 x 2000 x 100 BF16 24 and 12.
+// and of width 64 take 0.40 / 0.62 / 0.87 (BF16), 0.52 / 0.72 / 1.07 (split3)
+// and 0.75 / 1.05 / 1.42 (split6), about twice that where an operand has to be
+// read in pairs, and 5 per further wave of tiles; the two-pass contraction
+// 0.30 / 0.85 / 1.85 on its wider tiles, after a split pass at 4 TB/s and two
+// more launches.  Either side of the line, direct against two-pass: 64 x 4096
+// x 8192 BF16 56 and 86 us, split3 69 and 200, split6 100 and 351; 1024^3
+// split3 21 and 27, BF16 18 and 16; 512^3 BF16 9.5 and 12.8; 1000 x 777 x 1100
+// BF16 18 and 22; 1536^3 split3 54 and 37; 128 x 128 x 4096 BF16 39 and 28;
+// 64 x 4095 x 8191 BF16 (pairs) 127 and 103; 2000 x 2000 x 100 BF16 24 and 13.
 int direct_width(const gatlas_matmul_desc *d, const Geometry &g, const float *A, const float *B, const float *C) {
     using namespace direct;
     if (d->engine == GATLAS_ENGINE_TC_FP8) return 0;  // block scales need whole 128 x 128 blocks first
@@ -552,25 +553,25 @@ int direct_width(const gatlas_matmul_desc *d, const Geometry &g, const float *A,
     if (d->engine == GATLAS_ENGINE_TC_SPLIT6 && d->extra % 2 != 0) return 0;
     if (g.M > (1 << 20) || g.N > (1 << 20) || g.K > (1 << 24)) return 0;
     const int mode = d->engine == GATLAS_ENGINE_TC_BF16 ? 0 : d->engine == GATLAS_ENGINE_TC_SPLIT3 ? 1 : 2;
-    static const double kDirect[3][3] = {{0.40, 0.60, 0.80}, {0.52, 0.75, 1.05}, {0.75, 1.00, 1.40}};
-    static const double kTwoPass[3] = {0.30, 0.85, 1.85};
+    static const double kDirect[3][3] = {{0.40, 0.62, 0.87}, {0.52, 0.72, 1.07}, {0.75, 1.05, 1.42}};
+    static const double kPairs[3] = {2.2, 1.9, 1.45}, kTwoPass[3] = {0.30, 0.85, 1.85};
     const double sms = sm_count(), slices = (double)((g.K + kSlice - 1) / kSlice);
     auto waves = [](double tiles, double units) { return std::ceil(tiles / units); };
     auto tiles = [&](int64_t m, int64_t n) { return (double)((g.M + m - 1) / m) * (double)((g.N + n - 1) / n) * (double)g.batch; };
     const bool pairs = source(A, g.lda, g.M, g.stride_a, g.batch, g.ta).kind == kAlong ||
                        source(B, g.ldb, g.N, g.stride_b, g.batch, !g.tb).kind == kAlong;
     auto direct_us = [&](int bn) {
-        const double per_slice = kDirect[mode][g.M <= 64 ? 0 : bn == 32 ? 1 : 2] * (pairs ? 1.6 : 1.0);
+        const double per_slice = kDirect[mode][g.M <= 64 ? 0 : bn == 32 ? 1 : 2] * (pairs ? kPairs[mode] : 1.0);
         const double w = waves(tiles(128, bn), sms);
-        return 4.0 + w * slices * per_slice + (w - 1) * 1.5;
+        return 4.0 + w * slices * per_slice + (w - 1) * 5.0;
     };
     const bool pair = mode != 0 && g.M > BM;
     const double elems = (double)g.batch * (double)g.K * (double)(g.M + g.N);
-    // C by plain stores (beta, or rows not 16-byte aligned): 3 us per MB
+    // C by plain stores (beta, or rows not 16-byte aligned): 1 us per MB
     const bool plain_c = (d->gemm && d->beta != 0.0) || g.ldc % 4 != 0 || !aligned16(C) || (g.batch > 1 && g.stride_c % 4 != 0);
     const double two_pass_us = 9.0 + elems * (4 + 2 * (mode + 1)) / 4e6 +
                                waves(tiles(pair ? 256 : 128, 256), pair ? sms / 2 : sms) * slices * kTwoPass[mode] +
-                               (plain_c ? (double)g.batch * (double)g.M * (double)g.N * 4 * 3e-6 : 0.0);
+                               (plain_c ? (double)g.batch * (double)g.M * (double)g.N * 4 * 1e-6 : 0.0);
     const double us32 = direct_us(32), us64 = g.M <= 64 ? us32 : direct_us(64);
     if (std::min(us32, us64) > two_pass_us) return 0;
     return us32 <= us64 ? 32 : 64;

@@ -510,10 +510,12 @@ static int matvec_launch(const gatlas_matvec_desc *d, const T *A, const T *x, T 
     if (!d->trans_a) {
         constexpr int VWV = 16 / sizeof(T);
         const size_t per_row = vec_ok ? d->n / VWV : d->n;  // loads per row
-        if (per_row >= (size_t)4 * kGemvThreads) {
-            // long rows: a CTA per RB rows (see gemv_rowblock_kernel); elements
-            // of rows off the 16-byte grid are a quarter (half) as wide, so twice
-            // as many are in flight where the row holds that many
+        // long rows take a CTA per RB rows: 1024 vectors, or as many single elements
+        // unless there are rows enough for a warp each (27908 x 1287 doubles: 58 us
+        // with warps, 62 with CTAs; 3001 x 7013: 46 and 18)
+        const bool many = d->m * batch >= (size_t)sms * 64;
+        if (per_row >= (size_t)4 * kGemvThreads && (vec_ok || !many || per_row >= (size_t)16 * kGemvThreads)) {
+            // (single elements: twice as many in flight where the row holds them)
             constexpr int RB = 2;
             const size_t nblocks = (d->m + RB - 1) / RB;
             const size_t cap = (size_t)sms * 64 / (batch < 8 ? batch : 8);
