@@ -94,12 +94,15 @@ constexpr int grouped_seg_kblocks(int mode) { return mode == 0 ? tcg::kSegAll : 
 // kRowBytes; 16-byte chunk j of row r sits at chunk j ^ (r & 7) (128-byte
 // swizzle) or j ^ ((r >> 1) & 3) (64-byte swizzle), the layouts the MMA's
 // shared-memory descriptors read.
+// tr is a power of two (128 rows of A; 64, 128 or 256 of B): shifts, because a
+// 64-bit division per store was half of the pack pass's instructions.
 __device__ __forceinline__ int64_t packed_offset(int64_t row, int kb, int c, int tr, int kt) {
     constexpr int per = (int)(kRowBytes / 16);  // chunks per slice row
     const int s = kb * kSlicesPerItem + c / per, j = c % per;
     const int swz = kRowBytes == 128 ? (int)(row & 7) : (int)((row >> 1) & 3);
-    return ((row / tr) * (int64_t)(kt * kSlicesPerItem) + s) * (int64_t)tr * kRowBytes + (row % tr) * kRowBytes +
-           ((j ^ swz) << 4);
+    const int shift = 31 - __clz(tr);
+    return (((row >> shift) * (int64_t)(kt * kSlicesPerItem) + s) << shift) * kRowBytes +
+           (row & (tr - 1)) * kRowBytes + ((j ^ swz) << 4);
 }
 
 // ---------------------------------------------------------------------------
@@ -118,14 +121,13 @@ struct PackItem {
     bool transposed, vec;
 };
 
-__device__ __forceinline__ PackItem pack_item(const Inst *insts, const int64_t *seg_start, int sgi, int64_t it) {
+__device__ __forceinline__ PackItem pack_item(const Inst *insts, int sgi, int kb, int64_t rblock) {
     PackItem q;
     q.I = insts + (sgi >> 1);
     const Inst &I = *q.I;
     q.op = sgi & 1;
-    const int64_t local = it - seg_start[sgi];
-    q.kb = (int)(local % I.kt);
-    q.r0 = (local / I.kt) * kPackRows;
+    q.kb = kb;
+    q.r0 = rblock * kPackRows;
     q.k0 = (int64_t)q.kb * kPackBK;
     q.rows = q.op ? I.N : I.M;
     q.tr = q.op ? I.bn : BM;
@@ -137,6 +139,38 @@ __device__ __forceinline__ PackItem pack_item(const Inst *insts, const int64_t *
     q.K = I.K;
     return q;
 }
+
+// A place in the item space, advanced item by item without divisions.
+struct PackCursor {
+    const Inst *insts;
+    const int64_t *seg_start;
+    int64_t it, rblock;
+    int sgi, kb, kt;
+
+    // the item `at` of segment `sg` (at < seg_start[sg + 1])
+    __device__ __forceinline__ void place(const Inst *in, const int64_t *starts, int sg, int64_t at) {
+        insts = in, seg_start = starts, it = at, sgi = sg;
+        kt = insts[sgi >> 1].kt;
+        const int64_t local = it - seg_start[sgi];
+        rblock = local / kt;
+        kb = (int)(local - rblock * kt);
+    }
+    __device__ __forceinline__ PackItem item() const { return pack_item(insts, sgi, kb, rblock); }
+    // to the next item, which is before `end`, the end of this CTA's range
+    __device__ __forceinline__ void next(int64_t end) {
+        if (++it >= end) return;
+        if (++kb == kt) {
+            kb = 0;
+            ++rblock;
+            if (it >= seg_start[sgi + 1]) {
+                do ++sgi;
+                while (it >= seg_start[sgi + 1]);
+                kt = insts[sgi >> 1].kt;
+                rblock = 0;
+            }
+        }
+    }
+};
 
 // Stage layout: [128 rows][64 k] floats (rows of 256 B) for row-major
 // sources, [64 k][128 rows] (k rows of 512 B) for transposed ones, where the
@@ -167,26 +201,29 @@ __device__ __forceinline__ void cp_async_wait() {
 // copies (no registers held while they fly); bytes past M, N or K are
 // zero-filled by the copies themselves.
 __device__ __forceinline__ void pack_issue(const PackItem &q, uint8_t *stage, int tid) {
+    // stage[r][k]: 16 chunks per 256-byte row; transposed, stage[k][r]: 32 chunks
+    // per 512-byte k row.  A thread keeps its chunk along the row and takes
+    // every 16th row (8th k row).
+    const int o = q.transposed ? tid >> 5 : tid >> 4, ostep = q.transposed ? 8 : 16;
+    const int64_t outer = (q.transposed ? q.k0 : q.r0) + o;
+    const int64_t inner = q.transposed ? q.r0 + (tid & 31) * 4 : q.k0 + (tid & 15) * 4;
+    const int64_t left = (q.transposed ? q.rows : q.K) - inner, oleft = (q.transposed ? q.K : q.rows) - outer;
+    const int inside = left >= 4 ? 4 : (left > 0 ? (int)left : 0);
+    const float *p = q.src + outer * q.ld + inner;
+    const int64_t step = (int64_t)ostep * q.ld;
 #pragma unroll
     for (int j = 0; j < kPackChunks; ++j) {
-        const int e = j * 256 + tid;
-        int64_t outer, inner, outer_lim, inner_lim;
-        if (!q.transposed) {  // stage[r][k]: 16 chunks per 256-byte row
-            outer = q.r0 + (e >> 4), inner = q.k0 + (e & 15) * 4, outer_lim = q.rows, inner_lim = q.K;
-        } else {              // stage[k][r]: 32 chunks per 512-byte k row
-            outer = q.k0 + (e >> 5), inner = q.r0 + (e & 31) * 4, outer_lim = q.K, inner_lim = q.rows;
-        }
-        int64_t valid = outer < outer_lim ? inner_lim - inner : 0;
-        valid = valid < 0 ? 0 : (valid > 4 ? 4 : valid);
-        const float *src = valid > 0 ? q.src + outer * q.ld + inner : q.src;
-        uint8_t *dst = !q.transposed ? stage + (size_t)e * 16
-                                     : stage + (size_t)(e >> 5) * 512 + (((e & 31) ^ ((e >> 8) & 7)) << 4);
+        const int valid = j * ostep < oleft ? inside : 0;
+        const float *src = valid ? p : q.src;
+        uint8_t *dst = !q.transposed ? stage + (size_t)(j * 256 + tid) * 16
+                                     : stage + (size_t)(o + 8 * j) * 512 + (((tid & 31) ^ j) << 4);
         if (q.vec) {
             cp_async16(dst, src, (uint32_t)valid * 4);
         } else {
 #pragma unroll
             for (int v = 0; v < 4; ++v) cp_async4(dst + 4 * v, v < valid ? src + v : q.src, v < valid ? 4u : 0u);
         }
+        p += step;
     }
 }
 
@@ -218,15 +255,15 @@ __global__ void __launch_bounds__(256, 2) grouped_pack_kernel(const Inst *insts,
 
     // issue cursor: one commit group per item (empty past the range), so that
     // wait_group counts items
-    int psgi = sgi;
-    int64_t pit = it0;
+    PackCursor ahead, here;
+    ahead.place(insts, seg_start, sgi, it0);
+    here = ahead;
     auto issue_next = [&]() {
-        if (pit < it1) {
-            while (pit >= seg_start[psgi + 1]) ++psgi;
-            pack_issue(pack_item(insts, seg_start, psgi, pit), stage_of(pit), tid);
+        if (ahead.it < it1) {
+            pack_issue(ahead.item(), stage_of(ahead.it), tid);
+            ahead.next(it1);
         }
         cp_async_commit();
-        ++pit;
     };
     for (int i = 0; i < kPackStages - 1; ++i) issue_next();
 
@@ -234,8 +271,8 @@ __global__ void __launch_bounds__(256, 2) grouped_pack_kernel(const Inst *insts,
         issue_next();  // into the stage the previous iteration released
         cp_async_wait<kPackStages - 1>();  // this thread's copies of item `it` have landed
         __syncthreads();                   // and every other thread's
-        while (it >= seg_start[sgi + 1]) ++sgi;
-        const PackItem cur = pack_item(insts, seg_start, sgi, it);
+        const PackItem cur = here.item();
+        here.next(it1);
         const float *tile = reinterpret_cast<const float *>(stage_of(it));
         uint8_t *const *dst = cur.op ? cur.I->pb : cur.I->pa;
 #pragma unroll
