@@ -51,18 +51,24 @@ constexpr int kBK = kRowBytes / 2;        // BF16 elements per contraction K sli
 constexpr int kSlicesPerItem = (int)(kPackRowBytes / kRowBytes);
 constexpr uint32_t kATileBytes = BM * kRowBytes;
 constexpr int kDrainWarps = 8;            // a multiple of 4: kDrainParts warps per TMEM lane quarter
-constexpr int kThreads = 32 * (2 + kDrainWarps);
+// Roles are whole warpgroups: warps 0 and 1 produce and issue (2 and 3 idle),
+// warps 4..11 drain.  The first group gives its registers to the drain, whose
+// 128 sums, a chunk of C and the tile's record do not fit the 168 that 384
+// threads start with: 128 x 40 + 256 x 232 = 384 x 168.
+constexpr int kThreads = 32 * (4 + kDrainWarps);
+constexpr int kIssueRegs = 40, kDrainRegs = 232;
+static_assert(128 * kIssueRegs + 32 * kDrainWarps * kDrainRegs <= kThreads * 168, "register split");
 constexpr int kDrainParts = kDrainWarps / 4;          // column parts of a tile per lane quarter
-constexpr int kPartGroups = 256 / kDrainParts / 8;    // 8-column groups in a part of the widest tile
-constexpr int kAccRegs = 2 * kPartGroups * 4;         // accumulator registers per drain thread
+constexpr int kPartCols = 256 / kDrainParts;          // columns in a part of the widest tile
 constexpr uint32_t kTmemCols = 512;       // two accumulators of up to 256 columns
 constexpr uint64_t kWaitNs = 2000000000ull;
 constexpr int kPackRows = 128;            // rows per pack item
-constexpr int kEpiBatch = 8;              // 8-column groups of C loaded together by the epilogue
-static_assert(kDrainWarps % 4 == 0 && kPartGroups % kEpiBatch == 0, "drain layout");
-// The grouped engine stages 64-byte K slices (its packed tiles carry the
-// 64-byte swizzle), so that a ring of 48 KiB stages holds four split3 K slices
-// of a 128 x 256 tile, and promotes after the same K as the single-instance
+constexpr uint32_t kEpiTileBytes = 32 * 32 * 4;
+constexpr uint32_t kEpiBytes = kDrainWarps * kEpiTileBytes;
+static_assert(kDrainWarps % 4 == 0 && kPartCols % 32 == 0, "drain layout");
+// The grouped engine stages 128-byte K slices (its packed tiles carry the
+// 128-byte swizzle): the ring holds two split3 slices of a 128 x 256 tile (96
+// KiB each) or four BF16 ones, beside the drain's staging.  It promotes after the same K as the single-instance
 // engine (all of K for one-product BF16, 256 for split3), issuing the same
 // MMA sequence (16-deep K steps in order, the products of each in order), so
 // that each instance's result is bit-identical to it.
@@ -79,9 +85,10 @@ struct GLayout {
     static constexpr uint32_t A_TILE = BM * kRowBytes;
     static constexpr uint32_t B_TILE = BROWS * kRowBytes;
     static constexpr uint32_t STAGE_BYTES = MD::NP * (A_TILE + B_TILE);
-    static constexpr int FIT = (int)((226 * 1024 - 1024) / STAGE_BYTES);
+    static constexpr int FIT = (int)((226 * 1024 - 1024 - kEpiBytes) / STAGE_BYTES);
     static constexpr int STAGES = FIT < 8 ? FIT : 8;
-    static constexpr uint32_t SMEM_BYTES = STAGES * STAGE_BYTES + 1024;  // + alignment slack
+    static constexpr uint32_t EPI_OFFSET = STAGES * STAGE_BYTES;  // a 32 x 32 staging tile of C per drain warp
+    static constexpr uint32_t SMEM_BYTES = EPI_OFFSET + kEpiBytes + 1024;  // + alignment slack
     static_assert(STAGES >= 2, "grouped pipeline depth");
 };
 template <int MODE, bool PAIR>
@@ -337,12 +344,21 @@ struct Params {
 // The leader's MMAs commit to both CTAs' ring and accumulator barriers; both
 // CTAs' drain warps (each on its own 128 rows of TMEM) arrive on the leader's.
 //
-// VEC: every instance's C takes 8-byte vector accesses (even N and ldc, C
-// 8-byte aligned), so the epilogue is built without its scalar path.  That
-// path, even never taken, costs the epilogue registers and instruction
-// fetch: the contraction of the 1024-instance mix ran 2.08 ms (BF16) with
-// it and 1.67 ms without.
-template <int MODE, bool PAIR, bool VEC>
+// The epilogue bounds short-K tiles: C is read and written once per tile, and
+// what counts is how much of it a warp has in flight and how whole its lines
+// are.  Sums are kept a row per lane (32x32b reads) and go through a 4 KiB
+// staging tile per warp, so that each instruction moves VEC rows of a 32-column
+// chunk by VEC floats a lane, with all the chunk's reads of C (4 KiB a warp) in
+// flight together.  VEC is 4, 2 or 1: all instances' N, ldc and C are multiples
+// of it.  Before, reads and stores were 32-byte pieces of eight rows, two
+// floats a lane, or one at a time when N was odd.  Contraction only, BF16, 148
+// products of 1024 x N x 128, beta = 1, N = 1024 / 1022 / 1023: 273 -> 227, 320
+// -> 274, 1590 -> 325 us; with beta = 0 162 -> 147, 217 -> 222 (lines split
+// between rows bound it), 370 -> 235 us.  256 uneven products up to 2048: split3 180
+// -> 166, BF16 118 -> 103 us.
+template <int VEC> struct alignas(4 * VEC) Vec { float x[VEC]; };
+
+template <int MODE, bool PAIR, int VEC>
 __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_kernel(Params p) {
     using L = GLayoutOf<MODE, PAIR>;
     using MD = tcg::Mode<MODE>;
@@ -399,6 +415,7 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_kernel(Params p) {
     auto a_tile = [&](int s, int piece) { return smem + s * L::STAGE_BYTES + piece * L::A_TILE; };
     auto b_tile = [&](int s, int piece) { return smem + s * L::STAGE_BYTES + MD::NP * L::A_TILE + piece * L::B_TILE; };
 
+    if (warp < 4) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kIssueRegs));
     if (warp == 0) {
         // ---- producer: one bulk copy per piece tile (all lanes walk and wait,
         // one elected lane issues, as in the MMA warp) ----
@@ -542,45 +559,44 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_kernel(Params p) {
             }
         }
         __syncwarp();
-    } else {
+    } else if (warp >= 4) {
         // ---- drain + epilogue ----
-        const int quarter = warp & 3, part = (warp - 2) >> 2;
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kDrainRegs));
+        const int quarter = warp & 3, part = (warp - 4) >> 2;
         const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
         const int row_off = PAIR ? (int)rank * 128 : 0;  // a pair CTA's rows of the 256-row tile
         const uint32_t tempty_leader = PAIR ? tc::mapa_shared(smem_u32(&tempty[0]), 0) : 0u;
+        uint8_t *stage = smem + L::EPI_OFFSET + (warp - 4) * kEpiTileBytes;
+        const int vr = lane / (32 / VEC), vc = lane % (32 / VEC) * VEC;  // a lane's row and column of an access to C
         int seg = 0;
         bool ok = true;
         for (int t = t_begin; t < t_end && ok; ++t) {
-            const TileRec *R = p.tiles + t;
-            const int bn = R->bn, kt = R->kt;
-            const int hw = bn / kDrainParts;   // columns of this warp's part of the tile
+            const TileRec rec = p.tiles[t];
+            const int bn = rec.bn, kt = rec.kt;
+            const int hw = bn / kDrainParts;   // columns of this warp's part of the tile: 32, 64 or 128
             const int nseg = (kt + p.seg_kblocks - 1) / p.seg_kblocks;
-            // Accumulator fragments in the 16x256b layout: for row slab rs (TMEM
-            // lanes 16*rs .. 16*rs+15 of this warp's quarter) and column group
-            // cg (8 columns), acc[(rs*kPartGroups + cg)*4 + e] holds row
-            // 16*rs + lane/4 (e = 0, 1) or 16*rs + lane/4 + 8 (e = 2, 3), column
-            // 8*cg + 2*(lane%4) + (e & 1) of this warp's part of the tile.  Four
-            // neighbouring lanes then hold 32 contiguous bytes of one row of C,
-            // so each store request covers whole sectors of eight rows.
-            float acc[kAccRegs];
+            // acc[c]: row `lane` of this warp's 32, column c of its part
+            float acc[kPartCols];
 #pragma unroll
-            for (int j = 0; j < kAccRegs; ++j) acc[j] = 0.0f;
-            const int ngroups = hw >> 3;         // 8-column groups of this warp's part: 2 to kPartGroups
-            {
-                // C is read by the epilogue (beta != 0): pull this warp's rows
-                // of it into L2 while the tile's MMAs run
-                const int r = row_off + quarter * 32 + lane;
-                if (R->gemm && R->beta != 0.0f && r < R->rows) {
-                    const int left = R->cols - part * hw;
-                    const int ncols = left < hw ? left : hw;
-                    const char *row = reinterpret_cast<const char *>(R->C + (int64_t)r * R->ldc + part * hw);
-                    for (int off = 0; off < ncols * 4; off += 128)
-                        asm volatile("prefetch.global.L2 [%0];" ::"l"(row + off));
-                }
+            for (int j = 0; j < kPartCols; ++j) acc[j] = 0.0f;
+            const int row0 = row_off + quarter * 32;
+            const int left = rec.cols - part * hw;
+            const int ncols = left < hw ? left : hw;  // valid columns of this part (may be none)
+            const int nrows = rec.rows - row0 < 32 ? rec.rows - row0 : 32;
+            // without the gemm option 1 and 0: a sum that began at +0 is never -0, so 1 * sum + 0 is the sum
+            const float alpha = rec.gemm ? rec.alpha : 1.0f;
+            const float beta = rec.gemm && rec.beta != 0.0f ? rec.beta : 0.0f;
+            float *C = rec.C + (int64_t)row0 * rec.ldc + part * hw;
+            if (beta != 0.0f && lane < nrows) {
+                // C is read by the epilogue: pull this warp's rows of it into L2
+                // while the tile's MMAs run
+                const char *row = reinterpret_cast<const char *>(C + (int64_t)lane * rec.ldc);
+                for (int off = 0; off < ncols * 4; off += 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(row + off));
             }
             for (int sg = 0; sg < nseg; ++sg, ++seg) {
                 const int b = seg & 1;
-                if (!wait(&tfull[b], (uint32_t)(seg >> 1) & 1u, 2 * kWaitNs)) {
+                // the warp leaves together: it meets again below
+                if (!__all_sync(0xffffffffu, wait(&tfull[b], (uint32_t)(seg >> 1) & 1u, 2 * kWaitNs))) {
                     if (!abort_flag) report_fault(p.fault, kFaultTcEpilogueWait);
                     abort_flag = 1;
                     ok = false;
@@ -589,31 +605,13 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_kernel(Params p) {
                 tc::fence_after_sync();
                 const uint32_t col_base = tmem + lane_base + (uint32_t)(b * 256 + part * hw);
 #pragma unroll
-                for (int rs = 0; rs < 2; ++rs) {
-                    const uint32_t slab = col_base + ((uint32_t)(rs * 16) << 16);
-                    if (ngroups >= 4) {
-#pragma unroll
-                        for (int c = 0; c < kPartGroups / 4; ++c) {   // 32 columns per load
-                            if (c * 4 < ngroups) {
-                                uint32_t r[16];
-                                tc::tmem_ld_16x256b_x4(slab + (uint32_t)(c * 32), r);
-                                tc::tmem_ld_wait();
-#pragma unroll
-                                for (int j = 0; j < 16; ++j) {
-                                    const int idx = (rs * kPartGroups + c * 4) * 4 + j;
-                                    acc[idx] = __fadd_rn(acc[idx], __uint_as_float(r[j]));
-                                }
-                            }
-                        }
-                    } else {   // a 16-column part (64-wide tiles split four ways)
-                        uint32_t r[8];
-                        tc::tmem_ld_16x256b_x2(slab, r);
+                for (int c = 0; c < kPartCols; c += 16) {
+                    if (c < hw) {
+                        uint32_t r[16];
+                        tc::tmem_ld_32x32b_x16(col_base + (uint32_t)c, r);
                         tc::tmem_ld_wait();
 #pragma unroll
-                        for (int j = 0; j < 8; ++j) {
-                            const int idx = rs * kPartGroups * 4 + j;
-                            acc[idx] = __fadd_rn(acc[idx], __uint_as_float(r[j]));
-                        }
+                        for (int j = 0; j < 16; ++j) acc[c + j] = __fadd_rn(acc[c + j], __uint_as_float(r[j]));
                     }
                 }
                 tc::fence_before_sync();
@@ -623,58 +621,38 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_kernel(Params p) {
                     else tc::mbar_arrive_remote(tempty_leader + (uint32_t)(b * sizeof(uint64_t)));
                 }
             }
-            if (!ok || abort_flag) break;
-            const int left = R->cols - part * hw;
-            const int ncols = left < hw ? left : hw;  // valid columns of this part
-            const bool gemm = R->gemm != 0;
-            const float alpha = R->alpha, beta = gemm ? R->beta : 0.0f;
-            const bool vec_ok = ((R->ldc & 1) == 0) && ((reinterpret_cast<uintptr_t>(R->C) & 7) == 0) &&
-                                ((part * hw) % 2 == 0);
-            const int cl = 2 * (lane & 3);
+            if (__any_sync(0xffffffffu, !ok || abort_flag)) break;
+            // C by 32 x 32 chunks through the warp's staging tile (16-byte chunk j
+            // of row r at j ^ (r & 7)): read and written in whole 128-byte lines
 #pragma unroll
-            for (int rs = 0; rs < 2; ++rs) {
+            for (int c = 0; c < kPartCols; c += 32) {
+                if (c >= ncols || nrows <= 0) break;
+                float *at = C + (int64_t)vr * rec.ldc + c + vc;
+                const bool in = c + vc < ncols;  // N is a multiple of VEC: vectors are in or out
+                Vec<VEC> old[32 / VEC];
 #pragma unroll
-                for (int rr = 0; rr < 2; ++rr) {
-                    const int row = row_off + quarter * 32 + rs * 16 + (lane >> 2) + 8 * rr;
-                    if (row >= R->rows) continue;
-                    float *cp = R->C + (int64_t)row * R->ldc + part * hw;
-                    // kEpiBatch 8-column groups at a time: their loads of C
-                    // (beta != 0) are issued together, then their stores
+                for (int i = 0; i < 32 / VEC; ++i) old[i] = {};
+                if (beta != 0.0f) {
 #pragma unroll
-                    for (int g0 = 0; g0 < kPartGroups; g0 += kEpiBatch) {
-                        if (g0 >= ngroups) break;
-                        float2 c2[kEpiBatch];
-#pragma unroll
-                        for (int q = 0; q < kEpiBatch; ++q) {
-                            const int col = (g0 + q) * 8 + cl;
-                            c2[q] = make_float2(0.0f, 0.0f);
-                            if (beta != 0.0f && vec_ok && col + 1 < ncols)
-                                c2[q] = *reinterpret_cast<const float2 *>(cp + col);
-                        }
-#pragma unroll
-                        for (int q = 0; q < kEpiBatch; ++q) {
-                            const int col = (g0 + q) * 8 + cl;
-                            const int idx = (rs * kPartGroups + g0 + q) * 4 + 2 * rr;
-                            if (col >= ncols) continue;
-                            if (vec_ok && col + 1 < ncols) {
-                                float2 v;
-                                v.x = gemm ? __fmaf_rn(alpha, acc[idx], beta == 0.0f ? 0.0f : beta * c2[q].x)
-                                           : acc[idx];
-                                v.y = gemm ? __fmaf_rn(alpha, acc[idx + 1], beta == 0.0f ? 0.0f : beta * c2[q].y)
-                                           : acc[idx + 1];
-                                *reinterpret_cast<float2 *>(cp + col) = v;
-                            } else if constexpr (!VEC) {
-#pragma unroll
-                                for (int e = 0; e < 2; ++e) {
-                                    if (col + e < ncols) {
-                                        const float bc = beta == 0.0f ? 0.0f : beta * cp[col + e];
-                                        cp[col + e] = gemm ? __fmaf_rn(alpha, acc[idx + e], bc) : acc[idx + e];
-                                    }
-                                }
-                            }
-                        }
-                    }
+                    for (int i = 0; i < 32; i += VEC)
+                        if (in && i + vr < nrows)
+                            old[i / VEC] = *reinterpret_cast<const Vec<VEC> *>(at + i * rec.ldc);
                 }
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    *reinterpret_cast<float4 *>(stage + lane * 128 + ((j ^ (lane & 7)) << 4)) =
+                        make_float4(acc[c + 4 * j], acc[c + 4 * j + 1], acc[c + 4 * j + 2], acc[c + 4 * j + 3]);
+                __syncwarp();
+#pragma unroll
+                for (int i = 0; i < 32; i += VEC) {
+                    const int r = i + vr;
+                    Vec<VEC> v = *reinterpret_cast<const Vec<VEC> *>(
+                        stage + r * 128 + (((vc >> 2) ^ (r & 7)) << 4) + (vc & 3) * 4);
+#pragma unroll
+                    for (int e = 0; e < VEC; ++e) v.x[e] = __fmaf_rn(alpha, v.x[e], beta * old[i / VEC].x[e]);
+                    if (in && r < nrows) *reinterpret_cast<Vec<VEC> *>(at + i * rec.ldc) = v;
+                }
+                __syncwarp();  // the staging tile is read
             }
         }
     }
@@ -747,7 +725,7 @@ static int pair_units_cap() {
     int dev = 0;
     cudaGetDevice(&dev);
     if (cap_dev != dev) {
-        auto kern = grp::grouped_gemm_kernel<MODE, true, false>;
+        auto kern = grp::grouped_gemm_kernel<MODE, true, 1>;
         cap = sm_count() / 2;
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)grp::GLayoutOf<MODE, true>::SMEM_BYTES) == cudaSuccess) {
@@ -855,13 +833,12 @@ int grouped_build(int engine, const gatlas_grouped_instance *in, int32_t count, 
         if (rc) return rc;
     }
     t->pair = g_pair_mode.load() == 1;
-    // the vector-only epilogue serves the launch when every C takes 8-byte
-    // accesses: even N and ldc, 8-byte aligned base
-    t->vec = true;
+    // the widest access to C that every instance takes
+    uint64_t low = 0;  // bits set in any N, ldc or C (in floats)
     for (int i = 0; i < count; ++i)
         if (in[i].m > 0 && in[i].n > 0)
-            t->vec = t->vec && (t->ip[i].N % 2 == 0) && (t->ip[i].ldc % 2 == 0) &&
-                     ((reinterpret_cast<uintptr_t>(in[i].c) & 7) == 0);
+            low |= (uint64_t)t->ip[i].N | (uint64_t)t->ip[i].ldc | reinterpret_cast<uintptr_t>(in[i].c) >> 2;
+    t->vec = low & 1 ? 1 : low & 2 ? 2 : 4;
     const int step_m = t->pair ? 2 : 1;
     size_t off = 0;
     for (int i = 0; i < count; ++i) {
@@ -977,37 +954,32 @@ int grouped_launch_pack(const GroupedTables &t, const GroupedDevice &d, cudaStre
     return check_launch("grouped_pack_kernel");
 }
 
-// Shared-memory attributes of the four contraction kernels, once per device
-// (also before a graph capture, since attribute changes are not captured).
+// Shared-memory attributes of the contraction kernels, once per device (also
+// before a graph capture, since attribute changes are not captured).
+template <int MODE, bool PAIR>
+static cudaError_t grouped_gemm_attribute() {
+    const int bytes = (int)grp::GLayoutOf<MODE, PAIR>::SMEM_BYTES;
+    for (auto kern : {grp::grouped_gemm_kernel<MODE, PAIR, 1>, grp::grouped_gemm_kernel<MODE, PAIR, 2>,
+                      grp::grouped_gemm_kernel<MODE, PAIR, 4>}) {
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
 static int grouped_gemm_attributes() {
     static thread_local int attr_dev = -1;
     int dev = 0;
     cudaGetDevice(&dev);
     if (attr_dev == dev) return GATLAS_OK;
-    const cudaError_t e[8] = {
-        cudaFuncSetAttribute(grp::grouped_gemm_kernel<0, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)grp::GLayoutOf<0, false>::SMEM_BYTES),
-        cudaFuncSetAttribute(grp::grouped_gemm_kernel<1, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)grp::GLayoutOf<1, false>::SMEM_BYTES),
-        cudaFuncSetAttribute(grp::grouped_gemm_kernel<0, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)grp::GLayoutOf<0, true>::SMEM_BYTES),
-        cudaFuncSetAttribute(grp::grouped_gemm_kernel<1, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)grp::GLayoutOf<1, true>::SMEM_BYTES),
-        cudaFuncSetAttribute(grp::grouped_gemm_kernel<0, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)grp::GLayoutOf<0, false>::SMEM_BYTES),
-        cudaFuncSetAttribute(grp::grouped_gemm_kernel<1, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)grp::GLayoutOf<1, false>::SMEM_BYTES),
-        cudaFuncSetAttribute(grp::grouped_gemm_kernel<0, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)grp::GLayoutOf<0, true>::SMEM_BYTES),
-        cudaFuncSetAttribute(grp::grouped_gemm_kernel<1, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)grp::GLayoutOf<1, true>::SMEM_BYTES)};
-    for (cudaError_t x : e)
-        if (x != cudaSuccess) return set_error(GATLAS_ERR_CUDA, "grouped smem attribute: %s", cudaGetErrorString(x));
+    for (cudaError_t e : {grouped_gemm_attribute<0, false>(), grouped_gemm_attribute<1, false>(),
+                          grouped_gemm_attribute<0, true>(), grouped_gemm_attribute<1, true>()})
+        if (e != cudaSuccess) return set_error(GATLAS_ERR_CUDA, "grouped smem attribute: %s", cudaGetErrorString(e));
     attr_dev = dev;
     return GATLAS_OK;
 }
 
-template <int MODE, bool PAIR, bool VEC>
+template <int MODE, bool PAIR>
 static int launch_grouped(const GroupedTables &t, const GroupedDevice &d, cudaStream_t stream) {
     grp::Params prm;
     prm.tiles = d.tiles;
@@ -1028,21 +1000,18 @@ static int launch_grouped(const GroupedTables &t, const GroupedDevice &d, cudaSt
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = PAIR ? 1 : 0;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, grp::grouped_gemm_kernel<MODE, PAIR, VEC>, prm);
+    const auto kern = t.vec == 4   ? grp::grouped_gemm_kernel<MODE, PAIR, 4>
+                      : t.vec == 2 ? grp::grouped_gemm_kernel<MODE, PAIR, 2>
+                                   : grp::grouped_gemm_kernel<MODE, PAIR, 1>;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, prm);
     if (e != cudaSuccess) return set_error(GATLAS_ERR_CUDA, "grouped_gemm_kernel: %s", cudaGetErrorString(e));
     return check_launch("grouped_gemm_kernel");
 }
 
 int grouped_launch_contract(const GroupedTables &t, const GroupedDevice &d, cudaStream_t stream) {
     if (t.ntiles == 0) return GATLAS_OK;
-    if (t.vec) {
-        if (t.pair)
-            return t.mode == 1 ? launch_grouped<1, true, true>(t, d, stream) : launch_grouped<0, true, true>(t, d, stream);
-        return t.mode == 1 ? launch_grouped<1, false, true>(t, d, stream) : launch_grouped<0, false, true>(t, d, stream);
-    }
-    if (t.pair)
-        return t.mode == 1 ? launch_grouped<1, true, false>(t, d, stream) : launch_grouped<0, true, false>(t, d, stream);
-    return t.mode == 1 ? launch_grouped<1, false, false>(t, d, stream) : launch_grouped<0, false, false>(t, d, stream);
+    if (t.pair) return t.mode == 1 ? launch_grouped<1, true>(t, d, stream) : launch_grouped<0, true>(t, d, stream);
+    return t.mode == 1 ? launch_grouped<1, false>(t, d, stream) : launch_grouped<0, false>(t, d, stream);
 }
 
 struct GroupedPlan {
