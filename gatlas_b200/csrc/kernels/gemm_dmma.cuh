@@ -148,6 +148,7 @@ __global__ void __launch_bounds__(BM / WM *(BN / WN) * 32, BM *BN >= 64 * 32 ? 3
         asm volatile("cp.async.commit_group;" ::: "memory");
     }
 
+
     double acc[MI][NI][4];
 #pragma unroll
     for (int i = 0; i < MI; ++i)
@@ -190,13 +191,38 @@ __global__ void __launch_bounds__(BM / WM *(BN / WN) * 32, BM *BN >= 64 * 32 ? 3
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 
     double *C = a.C + (int64_t)blockIdx.z * a.stride_c;
-    const bool vec_c = (a.ldc % 2 == 0) && ((reinterpret_cast<uintptr_t>(C) & 15) == 0);
+    const bool reads_c = a.gemm && a.beta != 0.0;
+    // 16 rows of C at a time, all their reads in flight together (one at a time,
+    // 2048 x 2048 x 64 with beta = 0.5 ran 40 us, so 31); 16-byte
+    // accesses where every pair of columns of the tile is whole.
+    const bool vec_c =
+        a.ldc % 2 == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0 && (a.N % 2 == 0 || n0 + BN <= a.N);
 #pragma unroll
-    for (int i = 0; i < MI; ++i)
+    for (int i = 0; i < MI; ++i) {
+        double old[2][NI][2];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int64_t row = m0 + wm + i * 16 + h * 8 + g;
-            if (row >= a.M) continue;
+            const double *crow = C + row * a.ldc;
+#pragma unroll
+            for (int j = 0; j < NI; ++j) {
+                const int64_t col = n0 + wn + j * 8 + 2 * t;
+                old[h][j][0] = old[h][j][1] = 0.0;
+                if (!reads_c) continue;
+                if (vec_c) {
+                    if (row < a.M && col < a.N) {
+                        const double2 v = *reinterpret_cast<const double2 *>(crow + col);
+                        old[h][j][0] = v.x, old[h][j][1] = v.y;
+                    }
+                } else {
+                    if (row < a.M && col < a.N) old[h][j][0] = crow[col];
+                    if (row < a.M && col + 1 < a.N) old[h][j][1] = crow[col + 1];
+                }
+            }
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int64_t row = m0 + wm + i * 16 + h * 8 + g;
             double *crow = C + row * a.ldc;
 #pragma unroll
             for (int j = 0; j < NI; ++j) {
@@ -204,19 +230,18 @@ __global__ void __launch_bounds__(BM / WM *(BN / WN) * 32, BM *BN >= 64 * 32 ? 3
                 double v[2] = {acc[i][j][2 * h], acc[i][j][2 * h + 1]};
                 if (a.gemm) {
 #pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        const double bc = (a.beta == 0.0 || col + e >= a.N) ? 0.0 : a.beta * crow[col + e];
-                        v[e] = __fma_rn(a.alpha, v[e], bc);
-                    }
+                    for (int e = 0; e < 2; ++e)
+                        v[e] = __fma_rn(a.alpha, v[e], reads_c ? a.beta * old[h][j][e] : 0.0);
                 }
-                if (vec_c && col + 1 < a.N) {
-                    *reinterpret_cast<double2 *>(crow + col) = make_double2(v[0], v[1]);
+                if (vec_c) {
+                    if (row < a.M && col < a.N) *reinterpret_cast<double2 *>(crow + col) = make_double2(v[0], v[1]);
                 } else {
-                    if (col < a.N) crow[col] = v[0];
-                    if (col + 1 < a.N) crow[col + 1] = v[1];
+                    if (row < a.M && col < a.N) crow[col] = v[0];
+                    if (row < a.M && col + 1 < a.N) crow[col + 1] = v[1];
                 }
             }
         }
+    }
 }
 
 }  // namespace dmma

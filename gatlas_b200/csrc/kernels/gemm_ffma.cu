@@ -17,7 +17,7 @@ struct Large {
     static constexpr bool AHEAD = false;
 };
 struct Medium {
-    static constexpr int BM = 128, BN = 64, TM = 8, TN = 8, LM = 8, MINB = 2, STAGES = 4;
+    static constexpr int BM = 128, BN = 64, TM = 8, TN = 8, LM = 4, MINB = 2, STAGES = 4;
     static constexpr bool AHEAD = true;
 };
 struct Small {

@@ -19,10 +19,16 @@
 // registers (packing them by moves instead ran 29 TFLOP/s, scalar
 // multiply-adds 37, turning 43 at 3072 x 2560 x 2048).
 //
+// The epilogue reads C a batch of rows at a time (element by element, each
+// waited for, a product of 3584 x 3072 x 64 with beta = 0.5 ran 62 us, in
+// batches 42; 1024^3 66 -> 62, 2047 x 2049 x 255 80 -> 68).
+//
 // Measured, default point before and after: 1024^3 119 -> 62 us, 256^3 36 -> 8,
 // 1001 x 1003 x 999 190 -> 69, 3072 x 2560 x 2048 with B transposed 896 -> 752,
 // 8192 x 8192 x 2048 50.3 -> 54.2 TFLOP/s.
 #pragma once
+
+#include <type_traits>
 
 #include "../common.cuh"
 
@@ -256,33 +262,68 @@ __global__ void __launch_bounds__(BM / TM *(BN / TN), MINB) gemm_ffma_kernel(Arg
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 
     float *C = a.C + (int64_t)blockIdx.z * a.stride_c;
-    const bool vec_c = (a.ldc % 4 == 0) && ((reinterpret_cast<uintptr_t>(C) & 15) == 0);
+    const bool reads_c = a.gemm && a.beta != 0.0f;
+    // Rows of C in batches of 32 elements a thread, all of a batch's reads in
+    // flight together; 16-byte accesses where every group of four columns of the
+    // tile is whole.
+    const bool vec_c =
+        a.ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0 && (a.N % 4 == 0 || n0 + BN <= a.N);
+    float *Ct = C + m0 * a.ldc + n0;
+    const int mleft = (int)min(a.M - m0, (int64_t)BM), nleft = (int)min(a.N - n0, (int64_t)BN);
+    auto finish = [&](auto reads) {
+        constexpr bool READS = decltype(reads)::value;
+        constexpr int ROWS = TM < 32 / TN ? TM : 32 / TN;
 #pragma unroll
-    for (int i = 0; i < TM; ++i) {
-        const int64_t row = m0 + wm + micro<!TA, LM>(ly, i);
-        if (row >= a.M) continue;
-        float *crow = C + row * a.ldc;
+        for (int i0 = 0; i0 < TM; i0 += ROWS) {
+            float old[ROWS][TN];
+            if constexpr (READS) {
 #pragma unroll
-        for (int j = 0; j < TN; j += 4) {
-            float v[4];
+                for (int i = 0; i < ROWS; ++i) {
+                    const int row = wm + micro<!TA, LM>(ly, i0 + i);
+                    const float *crow = Ct + row * a.ldc;
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int64_t col = n0 + wn + micro<false, LN>(lx, j + e);
-                v[e] = acc[i][j + e];
-                if (a.gemm) v[e] = __fmaf_rn(a.alpha, v[e], (a.beta == 0.0f || col >= a.N) ? 0.0f : a.beta * crow[col]);
+                    for (int j = 0; j < TN; j += 4) {
+                        const int col = wn + micro<false, LN>(lx, j);
+                        if (vec_c) {
+                            if (row < mleft && col < nleft) {
+                                const float4 v = *reinterpret_cast<const float4 *>(crow + col);
+                                old[i][j] = v.x, old[i][j + 1] = v.y, old[i][j + 2] = v.z, old[i][j + 3] = v.w;
+                            }
+                        } else {
+#pragma unroll
+                            for (int e = 0; e < 4; ++e)
+                                if (row < mleft && col + e < nleft) old[i][j + e] = crow[col + e];
+                        }
+                    }
+                }
             }
-            const int64_t c0 = n0 + wn + micro<false, LN>(lx, j);
-            if (vec_c && c0 + 3 < a.N) {
-                *reinterpret_cast<float4 *>(crow + c0) = make_float4(v[0], v[1], v[2], v[3]);
-            } else {
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int64_t col = n0 + wn + micro<false, LN>(lx, j + e);
-                    if (col < a.N) crow[col] = v[e];
+            for (int i = 0; i < ROWS; ++i) {
+                const int row = wm + micro<!TA, LM>(ly, i0 + i);
+                float *crow = Ct + row * a.ldc;
+#pragma unroll
+                for (int j = 0; j < TN; j += 4) {
+                    const int col = wn + micro<false, LN>(lx, j);
+                    float v[4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        v[e] = acc[i0 + i][j + e];
+                        if (a.gemm) v[e] = __fmaf_rn(a.alpha, v[e], READS ? a.beta * old[i][j + e] : 0.0f);
+                    }
+                    if (vec_c) {
+                        if (row < mleft && col < nleft)
+                            *reinterpret_cast<float4 *>(crow + col) = make_float4(v[0], v[1], v[2], v[3]);
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 4; ++e)
+                            if (row < mleft && col + e < nleft) crow[col + e] = v[e];
+                    }
                 }
             }
         }
-    }
+    };
+    if (reads_c) finish(std::true_type{});
+    else finish(std::false_type{});
 }
 
 template <int BM, int BN, bool TA, bool TB, int STAGES>
