@@ -36,7 +36,8 @@ bool matmul_ffma_takes(const Geometry &g);
 int matmul_ffma(const gatlas_matmul_desc *d, const Geometry &g, const float *A, const float *B, float *C,
                 cudaStream_t stream);
 
-// image engine: SIMT math on TMA tensor-map tile loads (gemm_image.cu)
+// image engine: SIMT math on TMA tensor-map tile loads (gemm_image.cu); its
+// default point runs the two above where they are faster
 int matmul_image_f32(const gatlas_matmul_desc *d, const Geometry &g, const float *A, const float *B,
                      float *C, cudaStream_t stream);
 int matmul_image_f64(const gatlas_matmul_desc *d, const Geometry &g, const double *A, const double *B,

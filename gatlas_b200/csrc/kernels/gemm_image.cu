@@ -1,4 +1,6 @@
-// Image engine for matmul: SIMT math fed by TMA tensor-map tiles.
+// Image engine for matmul: SIMT math fed by TMA tensor-map tiles, at explicit
+// points; the default point runs whichever kernel is faster for its size (see
+// tensor_maps_better).
 //
 // Host side of gemm_image.cuh: tensor maps (3-D: inner dimension, rows,
 // packed instance; 128-byte swizzle for the tiles whose rows run along K),
@@ -76,12 +78,40 @@ int img_smem_bytes(int scalar, bool ta, bool tb, int gh, int gw, int bh, int bw)
     return (2 * (a_raw + b_raw) + (ta ? 0 : BK * PA) + (tb ? BK * PB : 0)) * es + 1024;  // + alignment slack
 }
 
+// Whether the operands' tensor maps would be accepted: 32-bit extents, strides
+// below 2^40 bytes.  A default point that they refuse stays refused.
+bool maps_fit(const Geometry &g, int es) {
+    const int64_t rows = 1ll << 32, bytes = 1ll << 40;
+    if (g.M > rows || g.N > rows || g.K > rows || g.lda >= bytes / es || g.ldb >= bytes / es) return false;
+    if (g.batch > 1)
+        return g.stride_a > 0 && g.stride_b > 0 && g.stride_a < bytes / es && g.stride_b < bytes / es;
+    return g.lda * (g.ta ? g.K : g.M) < bytes / es && g.ldb * (g.tb ? g.N : g.K) < bytes / es;
+}
+
+// The default point's kernel.  Every kernel of the library computes the same
+// multiply-add chain, so the default takes the faster one: the buffer engine's
+// (asynchronous copies, tile by size; FP64 tensor-core instruction for double)
+// wherever it was measured, 1024^3 62 us against 116, 200 x 1000 x 1500 40
+// against 169, 3072 x 2560 x 2048 with B transposed 749 against 821, double
+// 1024^3 85 against 239, except float products whose two operands both land
+// k-major (nothing to transpose), with a long K and 128 x 128 tiles that fill
+// the SMs evenly: there the tensor-map tiles are 2 to 6 % ahead (2680 x 2680 x
+// 2048 529 us against 565, 1016 x 2040 x 2048 196 against 200; but K = 512 58
+// against 54, and 480 uneven tiles, 3072 x 2560 x 2048, 691 against 649).
+bool tensor_maps_better(int scalar, const Geometry &g) {
+    if (scalar || !g.ta || g.tb || g.K < 1024) return false;
+    const int64_t tiles = ((g.M + 127) / 128) * ((g.N + 127) / 128) * g.batch;
+    const int64_t per_sm = (tiles + sm_count() - 1) / sm_count();
+    return (double)tiles >= 0.85 * (double)(per_sm * sm_count());
+}
+
 template <typename T>
 int matmul_image_impl(const gatlas_matmul_desc *d, const Geometry &g, const T *A, const T *B, T *C,
                       cudaStream_t stream) {
     const int scalar = sizeof(T) == 8 ? 1 : 0;
     int gh = (int)d->group_h, gw = (int)d->group_w, bh = (int)d->block_h, bw = (int)d->block_w;
-    if (gh == 0 && gw == 0 && bh == 0 && bw == 0) {
+    const bool defaulted = gh == 0 && gw == 0 && bh == 0 && bw == 0;
+    if (defaulted) {
         gh = gw = 16;
         bh = scalar ? 4 : 8;
         bw = scalar ? 4 : 8;
@@ -106,6 +136,13 @@ int matmul_image_impl(const gatlas_matmul_desc *d, const Geometry &g, const T *A
         return set_error(GATLAS_ERR_UNSUPPORTED,
                          "matmul image engine: operands need 16-byte aligned rows and bases (lda, ldb multiples of %d)",
                          per16);
+    if (defaulted && maps_fit(g, es) && !tensor_maps_better(scalar, g)) {
+        if constexpr (sizeof(T) == 8) {
+            if (matmul_dmma_takes(g)) return matmul_dmma(d, g, A, B, C, stream);
+        } else {
+            if (matmul_ffma_takes(g)) return matmul_ffma(d, g, A, B, C, stream);
+        }
+    }
     const int BK = scalar ? 16 : 32;
     const int BM = gh * bh, BN = gw * bw;
     const int64_t a_inner = g.ta ? g.M : g.K, a_rows = g.ta ? g.K : g.M;

@@ -41,6 +41,9 @@ size_t gatlas_last_error(char *buf, size_t len);
 /* Engines.  BUFFER and IMAGE are the reference's two kernel families
  * ("matmulbuffer", "matmulimage", ...); on B200 the image family loads its
  * operands with TMA tensor-map / bulk copies instead of texture fetches.
+ * Matmul's image engine does so at explicit points; with all of the point 0 it
+ * runs the faster of its own and the buffer engine's default kernel (same bits),
+ * and asks for 16-byte aligned operand rows either way.
  * The TC_* engines are tcgen05 tensor-core contractions (no reference
  * counterpart): BF16 operands with FP32 accumulation, FP32 operands split
  * into BF16 pieces (3 or 6 products), FP8 E4M3 with FP32 block scales. */
