@@ -414,20 +414,51 @@ static ClusterPlan cluster_plan(const gatlas_matvec_desc *d, bool vec_ok) {
     ClusterPlan c{0, 0, 0};
     const size_t batch = d->batch ? d->batch : 1;
     if (d->n == 0 || (sizeof(T) == 8 && !vec_ok)) return c;
-    // narrow blocks with more rows in flight, as long as clusters of them fit the
-    // GPU at once; wide ones beyond (float: 5296 x 14956 49.7 us narrow and 60.5
-    // wide, 16384^2 167 and 156), 4096 doubles, 2048 off the 16-byte grid
-    const bool narrow = d->m <= (!vec_ok ? 2048u : sizeof(T) == 8 ? 4096u : 96u * (unsigned)sm_count());
-    c.variant = narrow ? 0 : 1;
-    c.width = narrow ? 32 : (vec_ok ? 32 * (16 / sizeof(T)) : 64);
-    const size_t blocks = (d->m + c.width - 1) / c.width * batch;
-    if (blocks * 8 < (size_t)sm_count() || blocks / batch > 0x7fffffffu) return c;
-    // clusters of up to 8 CTAs, as many in all as are resident for certain: four
-    // CTAs per SM, three of the float kernels with 16 rows in flight (5596 x
-    // 19076 doubles 196 us with 704 CTAs, 135 with 528), each of 64 rows at least
-    const size_t resident = (size_t)sm_count() * (sizeof(T) == 4 && narrow ? 3 : 4);
+    const size_t sms = (size_t)sm_count();
+    const auto blocks_of = [&](size_t width) { return (d->m + width - 1) / width * batch; };
+    // CTAs that a cluster launch is sure to have resident, in tenths of an SM:
+    // with more, a second wave of clusters doubles the time.  Fewer than fit one
+    // by one, since a cluster needs its CTAs in one place (3456 x 22652 floats,
+    // 54 blocks: 64 us with 8 segments, 50 with 7).
+    size_t tenths = 40;
+    if (sizeof(T) == 4 && vec_ok) {
+        // 64 columns, 16 rows in flight, wherever clusters of them fill the GPU and
+        // fit it (1716 x 19132: 27 us, with 32 columns 34, with 128 36; 16384^2 155,
+        // 184 and 160; 6772 x 3024 13, 16 and 14); 32 columns where there are too
+        // few blocks of 64, or so many that clusters of two no longer fit but single
+        // CTAs of 32 columns do (14000 x 6000: 53 us, 64 columns 56); 128 beyond
+        // (30000 x 4000: 78 us, 64 columns 90)
+        const size_t fit = sms * 27 / 10;
+        const bool pairs = blocks_of(64) * 2 <= fit, singles = blocks_of(32) <= sms * 3;
+        if (blocks_of(64) * 32 < sms * 5 || (!pairs && singles)) c.variant = 0, c.width = 32;
+        else if (blocks_of(64) <= fit) c.variant = 2, c.width = 64;
+        else c.variant = 1, c.width = 128;
+        if (c.variant != 1) tenths = 27;
+    } else if (sizeof(T) == 4) {
+        // off the 16-byte grid: 32 columns with more rows in flight up to 2048
+        // columns, 64 beyond (2047 x 20001: 34 us and 38; 3001 x 7013 19 and 15)
+        const bool narrow = d->m <= 2048;
+        c.variant = narrow ? 0 : 1, c.width = narrow ? 32 : 64;
+        tenths = narrow ? 30 : 35;  // (5001 x 14003: 67 us with 40, 54 with 35)
+    } else {
+        // doubles: 32 columns up to 4096, and where blocks of 64 are too many for
+        // clusters of two but leave SMs with two CTAs beside others with three
+        // (26804 x 3376: 110 us with 32, 126 with 64; 30000 x 2000 98 and 82, 8700 x
+        // 1588 23 and 22, 4720 x 9744 62 and 60)
+        const bool narrow = d->m <= 4096 || (blocks_of(64) > 2 * sms && blocks_of(64) <= 3 * sms);
+        c.variant = narrow ? 0 : 1, c.width = narrow ? 32 : 64;
+    }
+    const size_t blocks = blocks_of(c.width);
+    if (blocks * 8 < sms || blocks / batch > 0x7fffffffu) return c;
+    // clusters of up to 8 CTAs, as many in all as are resident, each of 64 rows at
+    // least (5596 x 19076 doubles 196 us with 704 CTAs, 135 with 528)
+    const size_t resident = sms * tenths / 10;
     int nseg = 8;
     while (nseg > 1 && (blocks * (size_t)nseg > resident || (size_t)nseg * 64 > d->n)) --nseg;
+    // long segments on SMs with two and three CTAs: the general kernel's finer
+    // segments even out (doubles, 1450 x 31575: 79 us, 67 there; 1176 x 12000 31 and
+    // 28; 1176 x 8192 21 both)
+    if (sizeof(T) == 8 && nseg == 8 && blocks * 8 < 3 * sms && d->n >= 10240) return c;
     c.nseg = nseg;
     return c;
 }
@@ -455,8 +486,9 @@ static int launch_cluster(const GemvArgs &g, const ClusterPlan &cp, bool vec_ok,
     cudaError_t e;
     if constexpr (sizeof(T) == 4) {
         if (vec_ok)
-            e = cp.variant == 0 ? cudaLaunchKernelEx(&cfg, gvc::gemv_cols_cluster_kernel<T, true, 8, V, 16>, a)
-                                : cudaLaunchKernelEx(&cfg, gvc::gemv_cols_cluster_kernel<T, true, 32, V, 8>, a);
+            e = cp.variant == 0   ? cudaLaunchKernelEx(&cfg, gvc::gemv_cols_cluster_kernel<T, true, 8, V, 16>, a)
+                : cp.variant == 1 ? cudaLaunchKernelEx(&cfg, gvc::gemv_cols_cluster_kernel<T, true, 32, V, 8>, a)
+                                  : cudaLaunchKernelEx(&cfg, gvc::gemv_cols_cluster_kernel<T, true, 16, V, 16>, a);
         else
             e = cp.variant == 0 ? cudaLaunchKernelEx(&cfg, gvc::gemv_cols_cluster_kernel<T, false, 16, 2, 16>, a)
                                 : cudaLaunchKernelEx(&cfg, gvc::gemv_cols_cluster_kernel<T, false, 16, 4, 8>, a);
@@ -466,6 +498,11 @@ static int launch_cluster(const GemvArgs &g, const ClusterPlan &cp, bool vec_ok,
     }
     if (e != cudaSuccess) return set_error(GATLAS_ERR_CUDA, "gemv_cols_cluster_kernel: %s", cudaGetErrorString(e));
     return check_launch("gemv_cols_cluster_kernel");
+}
+
+bool matvec_buffer_scratchless(const gatlas_matvec_desc *d, size_t elem_bytes) {
+    if (!d->trans_a) return true;
+    return (elem_bytes == 4 ? cluster_plan<float>(d, true) : cluster_plan<double>(d, true)).nseg > 0;
 }
 
 template <typename T>

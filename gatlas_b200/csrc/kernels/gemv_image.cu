@@ -1,4 +1,5 @@
-// GEMV image engine: A streamed through shared memory by TMA tensor-map loads.
+// GEMV image engine: A streamed through shared memory by TMA tensor-map loads,
+// where that is faster than the buffer engine's kernels (see tiles_better).
 //
 // Reference: KernelMatvecImage<SCALAR,VL> (KernelMatvecImage.hpp:188-295)
 // reads A and b through read_imagef texture fetches, one work item per
@@ -341,11 +342,12 @@ __global__ void __launch_bounds__(kThreads, 1)
 struct ColSegments {
     int64_t ncb, nseg, seg_len;
     size_t part_bytes, cnt_bytes;  // both 0 when nseg == 1 (no partial sums)
+    double eff;                    // share of the SMs' time that the rounds use
 };
 
 // cc: columns per block, ts: bytes per element (partial sums are elements).
 ColSegments col_segments(int64_t M, int64_t N, int sms, int64_t cc, size_t ts) {
-    ColSegments s{(M + cc - 1) / cc, 1, 0, 0, 0};
+    ColSegments s{(M + cc - 1) / cc, 1, 0, 0, 0, 0.0};
     const int64_t max_seg = std::min<int64_t>((N + CR - 1) / CR, 256);
     double best = -1.0;
     for (int64_t cand = 1; cand <= max_seg; ++cand) {
@@ -356,6 +358,7 @@ ColSegments col_segments(int64_t M, int64_t N, int sms, int64_t cc, size_t ts) {
         const double eff = (double)(s.ncb * N) / ((double)sms * (double)rounds * (double)(len + 128));
         if (eff > best + 1e-3) {
             best = eff;
+            s.eff = eff * (double)M / (double)(s.ncb * cc);
             s.nseg = segs;
             s.seg_len = len;
         }
@@ -380,12 +383,44 @@ struct TmaType<double> {
 
 }  // namespace gvi
 
+// gemv.cu: whether the buffer engine's kernel for a product with 16-byte rows
+// needs no workspace
+bool matvec_buffer_scratchless(const gatlas_matvec_desc *d, size_t elem_bytes);
+
 size_t matvec_image_ws_bytes(const gatlas_matvec_desc *d, size_t elem_bytes) {
     using namespace gvi;
     if (!d || !d->trans_a || d->n == 0 || d->m == 0) return 0;
     const ColSegments s =
         col_segments((int64_t)d->m, (int64_t)d->n, sm_count(), 1024 / (int64_t)elem_bytes, elem_bytes);
     return s.part_bytes + s.cnt_bytes;
+}
+
+// Whether a tensor map of A would be accepted (32-bit extents, a stride below
+// 2^40 bytes): a product that it refuses stays refused.
+static bool map_fits(int64_t inner, int64_t rows, int64_t lda, size_t ts) {
+    return inner <= (1ll << 32) && rows <= (1ll << 32) && lda < (1ll << 40) / (int64_t)ts;
+}
+
+// The buffer engine's kernels run the small and the uneven products.  Tiles in
+// shared memory stream as fast as loads into registers or a little faster, but
+// one CTA per SM takes whole blocks of 16 rows (or segments of a column block),
+// so its rounds have to come out even and its start has to be paid off.
+//  * rows: blocks that fill 90 % of their rounds (doubles 85), and 250 MB (25100
+//    x 3768 doubles 119 us, buffer 146; 16684 x 3720 86 and 99; 4420 x 15408
+//    floats 46 and 55; but 2788 x 28672 floats 78 and 51, 6412 x 1820 14 and 11);
+//  * columns: doubles whose segments use 82 % of the SMs' time, from 500 MB (87 %
+//    from 380: 16164 x 6136 116 us, buffer 128; 1932 x 25208 65 and 70; but 19824 x
+//    3300 103 and 81, floats 12036 x 1448 18 and 12, 2020 x 5472 19 and 10).
+template <typename T>
+static bool tiles_better(const gatlas_matvec_desc *d, int64_t M, int64_t N, int sms) {
+    using namespace gvi;
+    const double bytes = (double)M * (double)N * sizeof(T);
+    if (!d->trans_a) {
+        const int64_t blocks = (M + RB - 1) / RB, rounds = (blocks + sms - 1) / sms;
+        return bytes >= 250e6 && (double)blocks >= (sizeof(T) == 8 ? 0.85 : 0.9) * (double)(rounds * sms);
+    }
+    return sizeof(T) == 8 && bytes >= 380e6 &&
+           col_segments(M, N, sms, Elem<T>::ROW, sizeof(T)).eff >= (bytes >= 500e6 ? 0.82 : 0.87);
 }
 
 template <typename T>
@@ -416,7 +451,16 @@ int matvec_image(const gatlas_matvec_desc *d, const T *A, const T *x, T *y, void
     const uint64_t dims[2] = {(uint64_t)inner, (uint64_t)(d->trans_a ? N : M)};
     const uint64_t strides[1] = {(uint64_t)lda * TS};
     const int sms = sm_count();
+    const bool plain = map_fits(inner, d->trans_a ? N : M, lda, TS) && !tiles_better<T>(d, M, N, sms) &&
+                       matvec_buffer_scratchless(d, TS);
+    const auto run_plain = [&]() {
+        gatlas_matvec_desc b = *d;
+        b.engine = GATLAS_ENGINE_BUFFER;
+        if constexpr (sizeof(T) == 4) return gatlas_matvec_f32(&b, A, x, y, nullptr, 0, stream);
+        else return gatlas_matvec_f64(&b, A, x, y, nullptr, 0, stream);
+    };
     if (!d->trans_a) {
+        if (plain) return run_plain();
         const uint32_t box[2] = {(uint32_t)ROW, RB};
         int rc = make_tensor_map(&tm, TmaType<T>::value, 2, const_cast<T *>(A), dims, strides, box,
                                  CU_TENSOR_MAP_SWIZZLE_NONE);
@@ -429,12 +473,15 @@ int matvec_image(const gatlas_matvec_desc *d, const T *A, const T *x, T *y, void
         gemv_rows_tma_kernel<T><<<grid, kThreads, smem, stream>>>(tm, a);
         return check_launch("gemv_rows_tma_kernel");
     }
+    const ColSegments seg = col_segments(M, N, sms, ROW, TS);
+    const int64_t ncb = seg.ncb, nseg = seg.nseg, seg_len = seg.seg_len;
+    if (nseg > 1 && ws && (ws_bytes < seg.part_bytes + seg.cnt_bytes || !aligned_to(ws, 256)))
+        return set_error(GATLAS_ERR_INVALID, "matvec: workspace too small or not 256-byte aligned");
+    if (plain) return run_plain();
     const uint32_t box[2] = {(uint32_t)ROW, CR};
     int rc = make_tensor_map(&tm, TmaType<T>::value, 2, const_cast<T *>(A), dims, strides, box,
                              CU_TENSOR_MAP_SWIZZLE_NONE);
     if (rc) return rc;
-    const ColSegments seg = col_segments(M, N, sms, ROW, TS);
-    const int64_t ncb = seg.ncb, nseg = seg.nseg, seg_len = seg.seg_len;
     T *partial = nullptr;
     unsigned *counters = nullptr;
     if (nseg > 1) {
@@ -442,8 +489,6 @@ int matvec_image(const gatlas_matvec_desc *d, const T *A, const T *x, T *y, void
         if (!ws) {
             ws = device_scratch(part_bytes + cnt_bytes);
             if (!ws) return set_error(GATLAS_ERR_NOMEM, "matvec: scratch");
-        } else if (ws_bytes < part_bytes + cnt_bytes || !aligned_to(ws, 256)) {
-            return set_error(GATLAS_ERR_INVALID, "matvec: workspace too small or not 256-byte aligned");
         }
         partial = static_cast<T *>(ws);
         counters = reinterpret_cast<unsigned *>(static_cast<char *>(ws) + part_bytes);
