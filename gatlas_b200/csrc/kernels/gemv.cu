@@ -103,11 +103,67 @@ __device__ __forceinline__ void row_tail(T (&acc)[ROWS], const V *const (&arow)[
     }
 }
 
+// One group of U strided vectors per row, all loads in flight together.
+template <int U, int STRIDE, typename T, typename V, int ROWS>
+__device__ __forceinline__ void row_group(T (&acc)[ROWS], const V *const (&arow)[ROWS], const V *x, size_t c) {
+    V av[ROWS][U], xv[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) xv[u] = __ldg(x + c + u * STRIDE);
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r)
+#pragma unroll
+        for (int u = 0; u < U; ++u) av[r][u] = __ldcs(arow[r] + c + u * STRIDE);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) acc[r] = dot_acc(acc[r], av[r][u], xv[u]);
+}
+
+// The rest of a row, up to U vectors a lane, as one group for the whole warp;
+// only the last of them can be past the row, and is then read as the row's last
+// vector and left out of the sums.  (Where some lanes held one more full group
+// than others, the warp paid for both groups in turn, and a CTA waited three
+// latencies for that warp instead of two: 8000 rows of 7200 floats ran 56 us, of
+// 7168 39.)
+template <int U, int STRIDE, typename T, typename V, int ROWS>
+__device__ __forceinline__ void row_last(T (&acc)[ROWS], const V *const (&arow)[ROWS], const V *x, size_t c, int rem) {
+    V av[ROWS][U], xv[U];
+    const bool in = (U - 1) * STRIDE < rem;
+    const int last = in ? (U - 1) * STRIDE : rem - 1;  // -1 and below: before c, inside the row all the same
+#pragma unroll
+    for (int u = 0; u < U; ++u) xv[u] = __ldg(x + c + (u < U - 1 ? u * STRIDE : last));
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r)
+#pragma unroll
+        for (int u = 0; u < U; ++u) av[r][u] = __ldcs(arow[r] + c + (u < U - 1 ? u * STRIDE : last));
+#pragma unroll
+    for (int u = 0; u < U - 1; ++u)
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) acc[r] = dot_acc(acc[r], av[r][u], xv[u]);
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) acc[r] = in ? dot_acc(acc[r], av[r][U - 1], xv[U - 1]) : acc[r];
+}
+
+// Vectors c, c + STRIDE, ... of a row, four at a time; `first` is the warp's
+// smallest c.
+template <int STRIDE, typename T, typename V, int ROWS>
+__device__ __forceinline__ void row_strided(T (&acc)[ROWS], const V *const (&arow)[ROWS], const V *x, size_t c,
+                                            size_t first, size_t nvec) {
+    for (; first + 31 + 3 * STRIDE < nvec; first += 4 * STRIDE, c += 4 * STRIDE) row_group<4, STRIDE>(acc, arow, x, c);
+    if (first >= nvec) return;
+    const int rem = (int)((int64_t)nvec - (int64_t)c);
+    const int left = (int)(nvec - first);  // at most 4 * STRIDE
+    if (left > 3 * STRIDE) row_last<4, STRIDE>(acc, arow, x, c, rem);
+    else if (left > 2 * STRIDE) row_last<3, STRIDE>(acc, arow, x, c, rem);
+    else if (left > STRIDE) row_last<2, STRIDE>(acc, arow, x, c, rem);
+    else row_last<1, STRIDE>(acc, arow, x, c, rem);
+}
+
 // FEW: few warps per SM, so the tail of a row loads at once (row_tail); with
-// many the plain remainder loop is shorter and its latencies overlap (32768 x
-// 1023: 29 us, 33 with row_tail; 1024^2 the other way round).
+// many its extra loads cost more (32768 x 1023: 29 us, 33 with row_tail; 1024^2
+// the other way round).
 template <typename T, int VW, int ROWS, int UNROLL, bool FEW>
-__global__ void __launch_bounds__(kGemvThreads)
+__global__ void __launch_bounds__(kGemvThreads, VW == 2 ? 5 : 0)
     gemv_rows_kernel(GemvArgs a) {
     using V = typename VecT<T, VW>::type;
     const int lane = threadIdx.x & 31;
@@ -131,28 +187,17 @@ __global__ void __launch_bounds__(kGemvThreads)
             arow[r] = reinterpret_cast<const V *>(A + row * a.lda);
         }
         (void)ldv;
-        size_t c = lane;
-        for (; c + (UNROLL - 1) * 32 < nvec; c += UNROLL * 32) {
-            V av[ROWS][UNROLL], xv[UNROLL];
-#pragma unroll
-            for (int u = 0; u < UNROLL; ++u) xv[u] = __ldg(x + c + u * 32);
-#pragma unroll
-            for (int r = 0; r < ROWS; ++r)
-#pragma unroll
-                for (int u = 0; u < UNROLL; ++u) av[r][u] = __ldcs(arow[r] + c + u * 32);
-#pragma unroll
-            for (int u = 0; u < UNROLL; ++u)
-#pragma unroll
-                for (int r = 0; r < ROWS; ++r) acc[r] = dot_acc(acc[r], av[r][u], xv[u]);
-        }
         if constexpr (FEW) {
+            size_t c = lane;
+            for (; c + (UNROLL - 1) * 32 < nvec; c += UNROLL * 32) row_group<UNROLL, 32>(acc, arow, x, c);
             if (c < nvec) row_tail<T, V, ROWS, UNROLL, 32>(acc, arow, x, c, nvec);
-        } else {
-            for (; c < nvec; c += 32) {
-                const V xv = __ldg(x + c);
-#pragma unroll
-                for (int r = 0; r < ROWS; ++r) acc[r] = dot_acc(acc[r], __ldcs(arow[r] + c), xv);
-            }
+        } else if constexpr (VW > 1) {
+            static_assert(UNROLL == 4, "row_strided");
+            row_strided<32>(acc, arow, x, lane, 0, nvec);
+        } else {  // (row_strided: 32768 x 1023 floats 29 -> 41 us)
+            size_t c = lane;
+            for (; c + (UNROLL - 1) * 32 < nvec; c += UNROLL * 32) row_group<UNROLL, 32>(acc, arow, x, c);
+            for (; c < nvec; c += 32) row_group<1, 32>(acc, arow, x, c);
         }
 #pragma unroll
         for (int r = 0; r < ROWS; ++r) {
@@ -170,6 +215,9 @@ __global__ void __launch_bounds__(kGemvThreads)
     }
 }
 
+// (With five CTAs per SM: 48 registers a thread, asked for where the compiler
+// takes a few more.)
+//
 // Long rows: a CTA owns RB rows at a time and all 256 threads stride across
 // each of them in 16-byte vectors (UNROLL per row in flight, x reused from
 // registers across the RB rows); the per-thread chains are combined by a
@@ -177,7 +225,7 @@ __global__ void __launch_bounds__(kGemvThreads)
 // memory.  The units are 8 times smaller than a warp's rows, so a 16384^2
 // product is thousands of CTAs and the last partial wave costs little.
 template <typename T, int VW, int RB, int UNROLL>
-__global__ void __launch_bounds__(kGemvThreads)
+__global__ void __launch_bounds__(kGemvThreads, VW == 4 ? 5 : 0)
     gemv_rowblock_kernel(GemvArgs a) {
     using V = typename VecT<T, VW>::type;
     __shared__ T red[RB][kGemvWarps];
@@ -199,28 +247,14 @@ __global__ void __launch_bounds__(kGemvThreads)
             const size_t row = (row0 + r < a.M) ? row0 + r : a.M - 1;  // clamp; result discarded
             arow[r] = reinterpret_cast<const V *>(A + row * a.lda);
         }
-        size_t c = threadIdx.x;
-        for (; c + (UNROLL - 1) * kGemvThreads < nvec; c += UNROLL * kGemvThreads) {
-            V av[RB][UNROLL], xv[UNROLL];
-#pragma unroll
-            for (int u = 0; u < UNROLL; ++u) xv[u] = __ldg(x + c + u * kGemvThreads);
-#pragma unroll
-            for (int r = 0; r < RB; ++r)
-#pragma unroll
-                for (int u = 0; u < UNROLL; ++u) av[r][u] = __ldcs(arow[r] + c + u * kGemvThreads);
-#pragma unroll
-            for (int u = 0; u < UNROLL; ++u)
-#pragma unroll
-                for (int r = 0; r < RB; ++r) acc[r] = dot_acc(acc[r], av[r][u], xv[u]);
-        }
         if constexpr (VW == 1) {
+            size_t c = threadIdx.x;
+            for (; c + (UNROLL - 1) * kGemvThreads < nvec; c += UNROLL * kGemvThreads)
+                row_group<UNROLL, kGemvThreads>(acc, arow, x, c);
             if (c < nvec) row_tail<T, V, RB, UNROLL, kGemvThreads>(acc, arow, x, c, nvec);
-        } else {  // (row_tail would cost the fifth CTA per SM its registers: 16 -> 21 us at 1272 x 16108)
-            for (; c < nvec; c += kGemvThreads) {
-                const V xv = __ldg(x + c);
-#pragma unroll
-                for (int r = 0; r < RB; ++r) acc[r] = dot_acc(acc[r], __ldcs(arow[r] + c), xv);
-            }
+        } else {
+            static_assert(UNROLL == 4, "row_strided");
+            row_strided<kGemvThreads>(acc, arow, x, threadIdx.x, w * 32, nvec);
         }
 #pragma unroll
         for (int r = 0; r < RB; ++r) {
@@ -549,8 +583,9 @@ static int matvec_launch(const gatlas_matvec_desc *d, const T *A, const T *x, T 
         const size_t per_row = vec_ok ? d->n / VWV : d->n;  // loads per row
         // long rows take a CTA per RB rows: 1024 vectors, or as many single elements
         // unless there are rows enough for a warp each (27908 x 1287 doubles: 58 us
-        // with warps, 62 with CTAs; 3001 x 7013: 46 and 18)
-        const bool many = d->m * batch >= (size_t)sms * 64;
+        // with warps, 62 with CTAs; 3001 x 7013: 46 and 18; 7001 x 1201 floats 9 and
+        // 10, doubles 19 and 17)
+        const bool many = d->m * batch >= (size_t)sms * (sizeof(T) == 4 && per_row < (size_t)8 * kGemvThreads ? 32 : 64);
         if (per_row >= (size_t)4 * kGemvThreads && (vec_ok || !many || per_row >= (size_t)16 * kGemvThreads)) {
             // (single elements: twice as many in flight where the row holds them)
             constexpr int RB = 2;
@@ -563,8 +598,14 @@ static int matvec_launch(const gatlas_matvec_desc *d, const T *A, const T *x, T 
             return check_launch("gemv_rowblock_kernel");
         }
         // shorter rows: a warp per two rows, or per row (and twice the loads of
-        // it in flight) while that leaves SMs with few warps
-        const bool few = d->m * batch < (size_t)sms * 4 * kGemvWarps;
+        // it in flight) while that leaves SMs with few warps: up to about one wave
+        // of it, five CTAs per SM, and again where two rows a warp just begin a
+        // second wave (N = 3500: M = 6200 13 us and 17 with two rows, 7400 22 and
+        // 19, 11000 28 and 25, 13000 32 and 36, 18000 51 and 43)
+        const size_t rows_all = d->m * batch, wave = 5 * kGemvWarps * (size_t)sms;
+        const bool few = rows_all < (size_t)sms * 4 * kGemvWarps ||
+                         (vec_ok && (rows_all * 20 <= wave * (sizeof(T) == 8 ? 21 : 23) ||
+                                     (rows_all > 2 * wave && rows_all * 10 <= wave * 24)));
         const int rows = few ? 1 : 2;
         const size_t warps_needed = (d->m + rows - 1) / rows;
         size_t grid = (warps_needed + kGemvWarps - 1) / kGemvWarps;

@@ -35,7 +35,10 @@ def test_columns_exact(cuda, dtype, M, N):
 
 
 @pytest.mark.parametrize("dtype", [np.float32, np.float64])
-@pytest.mark.parametrize("M,N", [(1, 4), (17, 4096), (2372, 1000), (9474, 64)])
+# a lane's vectors 1, 4, 5, 7 and 8 with warps that end inside a group, row counts
+# where a warp's rows change; long rows in whole and in part
+@pytest.mark.parametrize("M,N", [(1, 4), (17, 4096), (2372, 1000), (9474, 64), (6808, 516), (6812, 508), (11844, 260),
+                                 (14212, 132), (37, 7168), (37, 7200), (39, 8192), (41, 8196), (5, 20484)])
 def test_image_rows_exact(cuda, dtype, M, N):
     import torch
     rng = np.random.default_rng(M + N)
