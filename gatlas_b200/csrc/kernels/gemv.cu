@@ -151,7 +151,8 @@ __device__ __forceinline__ void row_strided(T (&acc)[ROWS], const V *const (&aro
                                             size_t first, size_t nvec) {
     for (; first + 31 + 3 * STRIDE < nvec; first += 4 * STRIDE, c += 4 * STRIDE) row_group<4, STRIDE>(acc, arow, x, c);
     if (first >= nvec) return;
-    const int rem = (int)((int64_t)nvec - (int64_t)c);
+    // the same small number twice: which form stays within 48 registers depends on the caller
+    const int rem = STRIDE == 32 ? (int)((int64_t)nvec - (int64_t)c) : (int)nvec - (int)c;
     const int left = (int)(nvec - first);  // at most 4 * STRIDE
     if (left > 3 * STRIDE) row_last<4, STRIDE>(acc, arow, x, c, rem);
     else if (left > 2 * STRIDE) row_last<3, STRIDE>(acc, arow, x, c, rem);
@@ -215,8 +216,10 @@ __global__ void __launch_bounds__(kGemvThreads, VW == 2 ? 5 : 0)
     }
 }
 
-// (With five CTAs per SM: 48 registers a thread, asked for where the compiler
-// takes a few more.)
+// Five CTAs per SM need 48 registers a thread (56: 16384^2 floats 166 -> 170 us,
+// 30000 x 4400 90 -> 95).  Rows of one group and a short rest pay 3 % for the
+// clamped last group (30000 x 4400 87 -> 90, one element at a time), rows that end
+// in three or four vectors gain up to 40 %.
 //
 // Long rows: a CTA owns RB rows at a time and all 256 threads stride across
 // each of them in 16-byte vectors (UNROLL per row in flight, x reused from
@@ -225,7 +228,7 @@ __global__ void __launch_bounds__(kGemvThreads, VW == 2 ? 5 : 0)
 // memory.  The units are 8 times smaller than a warp's rows, so a 16384^2
 // product is thousands of CTAs and the last partial wave costs little.
 template <typename T, int VW, int RB, int UNROLL>
-__global__ void __launch_bounds__(kGemvThreads, VW == 4 ? 5 : 0)
+__global__ void __launch_bounds__(kGemvThreads)
     gemv_rowblock_kernel(GemvArgs a) {
     using V = typename VecT<T, VW>::type;
     __shared__ T red[RB][kGemvWarps];
