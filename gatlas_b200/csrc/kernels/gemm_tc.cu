@@ -731,17 +731,29 @@ __global__ void __launch_bounds__(kThreads2, 1)
 // ---------------------------------------------------------------------------
 // split pass: FP32 -> NP BF16 pieces, K-major [batch][rows][Kp]
 // ---------------------------------------------------------------------------
-struct SplitArgs {
+struct SplitOperand {
     const float *src;
     int64_t rows, K, Kp, ld, src_stride;  // src element (r,k): src[r*ld + k] (direct) or src[k*ld + r] (transposed)
     __nv_bfloat16 *out[3];
     int64_t piece_stride;                 // elements per instance in each piece: rows*Kp
+    int64_t row_tiles;                    // transposed: 64-row tiles; 0: direct
+};
+
+// One launch splits one operand or both: CTAs [0, split) the first operand,
+// the others the second.  HBM bounds large products, the launches and a division
+// per run did small ones: with a launch per operand, one run a thread and 64-bit
+// divisions, both operands of 1024^3 took 4.8 us in split3 (3.4 now; stored
+// across k 5.8 and 4.3), of 4096^3 47 (42), of 8192^3 180 (161; across k 209
+// and 206).
+struct SplitArgs {
+    SplitOperand op[2];
+    int64_t split;
 };
 
 // Stores the NP pieces of 8 consecutive elements of one K-major row: one
 // 16-byte store per piece (Kp is a multiple of 8, so every run is aligned).
 template <int NP>
-__device__ __forceinline__ void store_pieces8(const SplitArgs &a, int64_t z, int64_t r, int64_t k, const float (&x)[8]) {
+__device__ __forceinline__ void store_pieces8(const SplitOperand &a, int64_t z, int64_t r, int64_t k, const float (&x)[8]) {
     __nv_bfloat16 pcs[8][3];
 #pragma unroll
     for (int e = 0; e < 8; ++e) split_value<NP>(x[e], pcs[e]);
@@ -757,29 +769,53 @@ __device__ __forceinline__ void store_pieces8(const SplitArgs &a, int64_t z, int
     }
 }
 
-// Source stored rows x K (element (r,k) at src[r*ld + k]): each thread
-// splits runs of 8 consecutive k, read as two 16-byte loads where aligned.
+// Source stored rows x K (element (r,k) at src[r*ld + k]): a CTA splits
+// kSplitRuns * 256 runs of 8 consecutive k, read as two 16-byte loads where
+// aligned, all of a thread's runs in flight together where every run is whole.
+constexpr int kSplitRuns = 2;
 template <int NP>
-__global__ void __launch_bounds__(256) split_direct_kernel(SplitArgs a) {
-    const int64_t runs_per_row = a.Kp / 8;
-    const int64_t total = a.rows * runs_per_row;
-    const int64_t z = blockIdx.y;
+__device__ __forceinline__ void split_direct(const SplitOperand &a, int64_t block, int64_t z) {
+    const uint32_t per_row = (uint32_t)(a.Kp / 8);
+    const int64_t total = a.rows * per_row, q0 = block * (kSplitRuns * 256);
+    const int64_t row0 = q0 / per_row;
+    const uint32_t run0 = (uint32_t)(q0 - row0 * per_row) + threadIdx.x;
     const float *src = a.src + z * a.src_stride;
     const bool vec = (a.ld % 4 == 0) && ((reinterpret_cast<uintptr_t>(src) & 15) == 0);
-    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < total; q += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t r = q / runs_per_row, k = (q % runs_per_row) * 8;
-        const float *ptr = src + r * a.ld + k;
-        float x[8];
-        if (vec && k + 7 < a.K) {
-            const float4 u = __ldcs(reinterpret_cast<const float4 *>(ptr));
-            const float4 v = __ldcs(reinterpret_cast<const float4 *>(ptr + 4));
-            x[0] = u.x, x[1] = u.y, x[2] = u.z, x[3] = u.w, x[4] = v.x, x[5] = v.y, x[6] = v.z, x[7] = v.w;
-        } else {
+    int64_t r[kSplitRuns], k[kSplitRuns];
+    float x[kSplitRuns][8];
 #pragma unroll
-            for (int e = 0; e < 8; ++e) x[e] = (k + e < a.K) ? ptr[e] : 0.0f;
-        }
-        store_pieces8<NP>(a, z, r, k, x);
+    for (int u = 0; u < kSplitRuns; ++u) {
+        const uint32_t run = run0 + u * 256;
+        r[u] = row0 + run / per_row;
+        k[u] = (int64_t)(run % per_row) * 8;
     }
+    if (vec && a.K % 8 == 0) {
+#pragma unroll
+        for (int u = 0; u < kSplitRuns; ++u) {
+            const float *ptr = src + min(r[u], a.rows - 1) * a.ld + k[u];
+            const float4 v = __ldcs(reinterpret_cast<const float4 *>(ptr));
+            const float4 w = __ldcs(reinterpret_cast<const float4 *>(ptr + 4));
+            x[u][0] = v.x, x[u][1] = v.y, x[u][2] = v.z, x[u][3] = v.w;
+            x[u][4] = w.x, x[u][5] = w.y, x[u][6] = w.z, x[u][7] = w.w;
+        }
+    } else {
+#pragma unroll
+        for (int u = 0; u < kSplitRuns; ++u) {
+            const float *ptr = src + min(r[u], a.rows - 1) * a.ld + k[u];
+            if (vec && k[u] + 7 < a.K) {
+                const float4 v = __ldcs(reinterpret_cast<const float4 *>(ptr));
+                const float4 w = __ldcs(reinterpret_cast<const float4 *>(ptr + 4));
+                x[u][0] = v.x, x[u][1] = v.y, x[u][2] = v.z, x[u][3] = v.w;
+                x[u][4] = w.x, x[u][5] = w.y, x[u][6] = w.z, x[u][7] = w.w;
+            } else {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) x[u][e] = (k[u] + e < a.K) ? ptr[e] : 0.0f;
+            }
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < kSplitRuns; ++u)
+        if (q0 + threadIdx.x + u * 256 < total) store_pieces8<NP>(a, z, r[u], k[u], x[u]);
 }
 
 // Source stored K x rows (element (r,k) at src[k*ld + r]): 64 x 64 tiles
@@ -787,11 +823,11 @@ __global__ void __launch_bounds__(256) split_direct_kernel(SplitArgs a) {
 // writes are 16-byte runs of 8 k, eight threads covering one 128-byte row
 // segment per piece.
 template <int NP>
-__global__ void __launch_bounds__(256) split_transpose_kernel(SplitArgs a) {
-    __shared__ float tile[64][65];  // [k][r]
+__device__ __forceinline__ void split_transposed(const SplitOperand &a, int64_t block, int64_t z,
+                                                 float (&tile)[64][65]) {  // [k][r]
     const int tid = threadIdx.x;
-    const int64_t r0 = (int64_t)blockIdx.x * 64, k0 = (int64_t)blockIdx.y * 64;
-    const int64_t z = blockIdx.z;
+    const uint32_t tile_index = (uint32_t)block, row_tiles = (uint32_t)a.row_tiles;  // of a 31-bit grid
+    const int64_t r0 = (int64_t)(tile_index % row_tiles) * 64, k0 = (int64_t)(tile_index / row_tiles) * 64;
     const float *src = a.src + z * a.src_stride;
     const bool vec = (a.ld % 4 == 0) && ((reinterpret_cast<uintptr_t>(src) & 15) == 0);
 #pragma unroll
@@ -825,6 +861,17 @@ __global__ void __launch_bounds__(256) split_transpose_kernel(SplitArgs a) {
             store_pieces8<NP>(a, z, r, k, x);
         }
     }
+}
+
+// (Three pieces: 32 registers keep eight CTAs per SM, 8192^3 across k 276 -> 247 us.)
+template <int NP>
+__global__ void __launch_bounds__(256, NP == 3 ? 8 : 0) split_kernel(const __grid_constant__ SplitArgs a) {
+    __shared__ float tile[64][65];
+    const bool second = (int64_t)blockIdx.x >= a.split;
+    const SplitOperand &op = a.op[second ? 1 : 0];
+    const int64_t block = (int64_t)blockIdx.x - (second ? a.split : 0);
+    if (op.row_tiles) split_transposed<NP>(op, block, blockIdx.y, tile);
+    else split_direct<NP>(op, block, blockIdx.y);
 }
 
 // ---------------------------------------------------------------------------
@@ -1060,10 +1107,9 @@ static int launch_quant(const QuantOperand &first, const QuantOperand *second, i
     return check_launch("quant_fp8_kernel");
 }
 
-static int launch_split(int np, bool transposed, const float *src, int64_t rows, int64_t K, int64_t Kp,
-                        int64_t ld, int64_t src_stride, int64_t batch, __nv_bfloat16 *const out[3],
-                        cudaStream_t stream) {
-    SplitArgs a;
+static SplitOperand split_operand(bool transposed, const float *src, int64_t rows, int64_t K, int64_t Kp, int64_t ld,
+                                  int64_t src_stride, __nv_bfloat16 *const out[3]) {
+    SplitOperand a;
     a.src = src;
     a.rows = rows;
     a.K = K;
@@ -1072,24 +1118,33 @@ static int launch_split(int np, bool transposed, const float *src, int64_t rows,
     a.src_stride = src_stride;
     for (int i = 0; i < 3; ++i) a.out[i] = out[i];
     a.piece_stride = rows * Kp;
-    if (!transposed) {
-        const int64_t total = rows * (Kp / 8);
-        int64_t grid = (total + 255) / 256;
-        const int64_t cap = (int64_t)sm_count() * 16;
-        if (grid > cap) grid = cap;
-        dim3 gr((unsigned)(grid > 0 ? grid : 1), (unsigned)batch);
-        if (np == 1) split_direct_kernel<1><<<gr, 256, 0, stream>>>(a);
-        else if (np == 2) split_direct_kernel<2><<<gr, 256, 0, stream>>>(a);
-        else split_direct_kernel<3><<<gr, 256, 0, stream>>>(a);
-    } else {
-        const int64_t gx = (rows + 63) / 64, gy = (Kp + 63) / 64;
-        if (gy > 65535) return set_error(GATLAS_ERR_INVALID, "matmul: K too large for the transposing split");
-        dim3 gr((unsigned)gx, (unsigned)gy, (unsigned)batch);
-        if (np == 1) split_transpose_kernel<1><<<gr, 256, 0, stream>>>(a);
-        else if (np == 2) split_transpose_kernel<2><<<gr, 256, 0, stream>>>(a);
-        else split_transpose_kernel<3><<<gr, 256, 0, stream>>>(a);
-    }
-    return check_launch("split kernel");
+    a.row_tiles = transposed ? (rows + 63) / 64 : 0;
+    return a;
+}
+
+// Splits `first` and, when not null, `second` in one launch.
+static int launch_split(int np, const SplitOperand &first, const SplitOperand *second, int64_t batch,
+                        cudaStream_t stream) {
+    auto blocks = [](const SplitOperand &o) {
+        if (o.row_tiles) return o.row_tiles * ((o.Kp + 63) / 64);
+        const int64_t per_block = kSplitRuns * 256;
+        return (o.rows * (o.Kp / 8) + per_block - 1) / per_block;
+    };
+    for (const SplitOperand *o : {&first, second})
+        if (o && o->row_tiles && (o->Kp + 63) / 64 > 65535)
+            return set_error(GATLAS_ERR_INVALID, "matmul: K too large for the transposing split");
+    SplitArgs a;
+    a.op[0] = first;
+    a.op[1] = second ? *second : first;
+    a.split = blocks(first);
+    const int64_t total = a.split + (second ? blocks(*second) : 0);
+    if (total == 0) return GATLAS_OK;
+    if (total > 0x7fffffff) return set_error(GATLAS_ERR_INVALID, "matmul: operands too large for the split pass");
+    const dim3 gr((unsigned)total, (unsigned)batch);
+    if (np == 1) split_kernel<1><<<gr, 256, 0, stream>>>(a);
+    else if (np == 2) split_kernel<2><<<gr, 256, 0, stream>>>(a);
+    else split_kernel<3><<<gr, 256, 0, stream>>>(a);
+    return check_launch("split_kernel");
 }
 
 // Operand pointers inside a prepared workspace: [A pieces][B pieces], then
@@ -1413,9 +1468,8 @@ int tc_prepare(const gatlas_matmul_desc *d, const Geometry &g, const float *A, c
         ap[i] = static_cast<__nv_bfloat16 *>(w.a[i]);
         bp[i] = static_cast<__nv_bfloat16 *>(w.b[i]);
     }
-    rc = launch_split(pl.np, g.ta, A, g.M, g.K, pl.Kp, g.lda, g.stride_a, g.batch, ap, stream);
-    if (rc) return rc;
-    return launch_split(pl.np, !g.tb, B, g.N, g.K, pl.Kp, g.ldb, g.stride_b, g.batch, bp, stream);
+    const SplitOperand b = split_operand(!g.tb, B, g.N, g.K, pl.Kp, g.ldb, g.stride_b, bp);
+    return launch_split(pl.np, split_operand(g.ta, A, g.M, g.K, pl.Kp, g.lda, g.stride_a, ap), &b, g.batch, stream);
 }
 
 int tc_run(const gatlas_matmul_desc *d, const Geometry &g, const void *ws, size_t ws_bytes, float *C,
@@ -1457,7 +1511,7 @@ static int prepare_a_rows(const Plan &pl, const Geometry &g, const float *A, int
     __nv_bfloat16 *ap[3];
     for (int i = 0; i < 3; ++i)
         ap[i] = w.a[i] ? static_cast<__nv_bfloat16 *>(w.a[i]) + r0 * pl.Kp : nullptr;
-    return launch_split(pl.np, g.ta, src, rows, g.K, pl.Kp, g.lda, 0, 1, ap, s);
+    return launch_split(pl.np, split_operand(g.ta, src, rows, g.K, pl.Kp, g.lda, 0, ap), nullptr, 1, s);
 }
 
 static int prepare_b(const Plan &pl, const Geometry &g, const float *B, const WsPtrs &w, cudaStream_t s) {
@@ -1466,7 +1520,7 @@ static int prepare_b(const Plan &pl, const Geometry &g, const float *B, const Ws
                             nullptr, 1, s);
     __nv_bfloat16 *bp[3];
     for (int i = 0; i < 3; ++i) bp[i] = static_cast<__nv_bfloat16 *>(w.b[i]);
-    return launch_split(pl.np, !g.tb, B, g.N, g.K, pl.Kp, g.ldb, 0, 1, bp, s);
+    return launch_split(pl.np, split_operand(!g.tb, B, g.N, g.K, pl.Kp, g.ldb, 0, bp), nullptr, 1, s);
 }
 
 // Contracts rows [r0, r1) of A against all of B into rows [r0, r1) of C.
