@@ -222,7 +222,7 @@ int gatlas_matmul_f32_host(const gatlas_matmul_desc *d, const float *A, const fl
  * blocks two at a time, each CTA staging half of the B tile; the second half
  * of an odd instance's last pair is computed and not stored).  Results are
  * bit-identical.  On the 1024-instance log-uniform mix pairs are slower
- * (split3 3.9 vs 3.5 ms, BF16 3.0 vs 2.3 ms).  Read when a plan is created. */
+ * (split3 2.8 vs 2.5 ms, BF16 2.9 vs 1.3 ms).  Read when a plan is created. */
 int gatlas_set_option(const char *name, int64_t value);
 int gatlas_get_option(const char *name, int64_t *value);
 
