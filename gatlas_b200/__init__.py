@@ -120,6 +120,8 @@ def lib() -> ctypes.CDLL:
     L.gatlas_matmul_f32_host.argtypes = [ctypes.POINTER(MatmulDesc), vp, vp, vp, vp]
     L.gatlas_set_option.argtypes = [ctypes.c_char_p, ctypes.c_int64]
     L.gatlas_selftest_bounded_wait.argtypes = [ctypes.c_int64, ctypes.c_int, ctypes.POINTER(ctypes.c_int), vp]
+    L.gatlas_selftest_warp_wait.argtypes = [ctypes.c_int64, ctypes.POINTER(ctypes.c_int),
+                                            ctypes.POINTER(ctypes.c_int), vp]
     L.gatlas_get_option.argtypes = [ctypes.c_char_p, ctypes.POINTER(ctypes.c_int64)]
     gi = ctypes.POINTER(GroupedInstance)
     L.gatlas_grouped_workspace_size.argtypes = [i32, gi, ctypes.c_int32]
@@ -593,3 +595,12 @@ def selftest_bounded_wait(limit_ns=1_000_000, arrive=False, stream=None) -> bool
     s = None if stream is None else _stream(stream)  # NULL: the legacy default stream
     check(lib().gatlas_selftest_bounded_wait(int(limit_ns), int(bool(arrive)), ctypes.byref(done), s))
     return done.value == 1
+
+
+def selftest_warp_wait(limit_ns=200_000_000, stream=None):
+    """A whole warp's bounded wait whose lanes would decide differently by
+    themselves; (lanes told it completed, lanes elected afterwards)."""
+    done, elected = ctypes.c_int(-1), ctypes.c_int(-1)
+    s = None if stream is None else _stream(stream)
+    check(lib().gatlas_selftest_warp_wait(int(limit_ns), ctypes.byref(done), ctypes.byref(elected), s))
+    return done.value, elected.value

@@ -3,6 +3,7 @@
 
 #include "common.cuh"
 #include "device_state.cuh"
+#include "tcgen05.cuh"
 
 namespace gatlas {
 
@@ -140,6 +141,38 @@ __global__ void selftest_wait_kernel(int *fault, uint64_t limit_ns, int arrive, 
     *result = ok ? 1 : 0;
 }
 
+// A warp waits as the tensor-core kernels' warps do, with lanes that would
+// decide differently by themselves: half of them give up after limit_ns / 4, the
+// phase completes after limit_ns / 2 and the others would still wait then.
+// result[0]: lanes that were told the wait succeeded, result[1]: lanes elected
+// afterwards by the warp-wide instruction that MMAs are issued under.
+__global__ void selftest_warp_wait_kernel(int *fault, uint64_t limit_ns, int *result) {
+    __shared__ __align__(8) uint64_t bar;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        mbar_init(&bar, 1);
+        fence_mbarrier_init();
+    }
+    __syncthreads();
+    if (warp == 1) {
+        if (lane == 0) {
+            const uint64_t t0 = tc::globaltimer();
+            while (tc::globaltimer() - t0 < limit_ns / 2) {
+            }
+            mbar_arrive(&bar);
+        }
+        return;
+    }
+    const bool ok = tc::wait_warp(&bar, 0, lane < 16 ? limit_ns / 4 : limit_ns, nullptr);
+    if (!ok && lane == 0) report_fault(fault, kFaultSelftestWait);
+    const int done = __popc(__ballot_sync(0xffffffffu, ok));
+    const int elected = __popc(__ballot_sync(0xffffffffu, tc::elect_one()));
+    if (lane == 0) {
+        result[0] = done;
+        result[1] = elected;
+    }
+}
+
 }  // namespace
 }  // namespace gatlas
 
@@ -156,5 +189,24 @@ extern "C" int gatlas_selftest_bounded_wait(int64_t limit_ns, int arrive, int *c
     if (cudaMemcpyAsync(completed, res, sizeof(int), cudaMemcpyDeviceToHost, (cudaStream_t)stream) != cudaSuccess ||
         cudaStreamSynchronize((cudaStream_t)stream) != cudaSuccess)
         return check_launch("selftest result");
+    return GATLAS_OK;
+}
+
+extern "C" int gatlas_selftest_warp_wait(int64_t limit_ns, int *completed, int *elected, void *stream) {
+    using namespace gatlas;
+    if (limit_ns <= 0 || limit_ns > 2000000000LL || !completed || !elected)
+        return set_error(GATLAS_ERR_INVALID, "selftest: limit must be in (0, 2 s] and the results non-null");
+    int *fault = device_fault_word();
+    int *res = static_cast<int *>(device_scratch(2 * sizeof(int), 1));
+    if (!fault || !res) return set_error(GATLAS_ERR_NOMEM, "selftest: device words");
+    selftest_warp_wait_kernel<<<1, 64, 0, (cudaStream_t)stream>>>(fault, (uint64_t)limit_ns, res);
+    int rc = check_launch("selftest_warp_wait_kernel");
+    if (rc) return rc;
+    int host[2] = {-1, -1};
+    if (cudaMemcpyAsync(host, res, sizeof(host), cudaMemcpyDeviceToHost, (cudaStream_t)stream) != cudaSuccess ||
+        cudaStreamSynchronize((cudaStream_t)stream) != cudaSuccess)
+        return check_launch("selftest result");
+    *completed = host[0];
+    *elected = host[1];
     return GATLAS_OK;
 }

@@ -203,9 +203,9 @@ __global__ void __launch_bounds__(kThreadsP, 1)
         tm = first_m + r % gm;
         tn = r / gm;
     };
-    auto wait = [&](uint64_t *bar, uint32_t parity, uint64_t limit) {
-        return PAIR ? tc::wait_timed_cluster(bar, parity, limit, &abort_flag)
-                    : tc::wait_timed(bar, parity, limit, &abort_flag);
+    auto wait = [&](uint64_t *bar, uint32_t parity, uint64_t limit) {  // by whole warps
+        return PAIR ? tc::wait_warp_cluster(bar, parity, limit, &abort_flag)
+                    : tc::wait_warp(bar, parity, limit, &abort_flag);
     };
 
     if (threadIdx.x == 0) {
@@ -261,8 +261,10 @@ __global__ void __launch_bounds__(kThreadsP, 1)
             const int nb = tn * BN + (int)rank * (PAIR ? 128 : 0);
             for (int kb = 0; kb < p.kblocks; ++kb) {
                 if (!wait(&empty[s], ph ^ 1u, kWaitNs)) {
-                    if (lane == 0 && !abort_flag) report_fault(p.fault, kFaultTcProducerWait);
-                    abort_flag = 1;
+                    if (lane == 0) {
+                        if (!abort_flag) report_fault(p.fault, kFaultTcProducerWait);
+                        abort_flag = 1;
+                    }
                     stop = true;
                     break;
                 }
@@ -339,8 +341,10 @@ __global__ void __launch_bounds__(kThreadsP, 1)
                     // the drain of this buffer's previous segment (both CTAs' for a pair) is done
                     if ((seg_first && !wait(&tempty[b], ((uint32_t)(seg >> 1) & 1u) ^ 1u, kWaitNs)) ||
                         !wait(&full[s], ph, kWaitNs)) {
-                        if (lane == 0 && !abort_flag) report_fault(p.fault, kFaultTcMmaWait);
-                        abort_flag = 1;
+                        if (lane == 0) {
+                            if (!abort_flag) report_fault(p.fault, kFaultTcMmaWait);
+                            abort_flag = 1;
+                        }
                         stop = true;
                         break;
                     }
@@ -453,7 +457,7 @@ __global__ void __launch_bounds__(kThreadsP, 1)
                     else tc::mbar_arrive_remote(tempty_leader + (uint32_t)(b * sizeof(uint64_t)));
                 }
             }
-            if (!ok || abort_flag) break;
+            if (__any_sync(0xffffffffu, !ok || abort_flag)) break;
             const int64_t row0 = m0 + quarter * 32;
             const int64_t col0 = n0 + half * (BN / 2);
             if (p.tma_store) {
@@ -588,9 +592,11 @@ __global__ void __launch_bounds__(kThreads2, 1)
             int tm, tn, z;
             decode(t, tm, tn, z);
             for (int kb = 0; kb < p.kblocks; ++kb) {
-                if (!tc::wait_timed(&empty[s], ph ^ 1u, kWaitNs, &abort_flag)) {
-                    if (lane == 0 && !abort_flag) report_fault(p.fault, kFaultTcProducerWait);
-                    abort_flag = 1;
+                if (!tc::wait_warp(&empty[s], ph ^ 1u, kWaitNs, &abort_flag)) {
+                    if (lane == 0) {
+                        if (!abort_flag) report_fault(p.fault, kFaultTcProducerWait);
+                        abort_flag = 1;
+                    }
                     stop = true;
                     break;
                 }
@@ -616,10 +622,12 @@ __global__ void __launch_bounds__(kThreads2, 1)
         for (int64_t t = unit; t < total && !stop; t += units, tph ^= 1u) {
             for (int kb = 0; kb < p.kblocks; ++kb) {
                 // the drain has read the previous tile's accumulators, the slice has landed
-                if ((kb == 0 && !tc::wait_timed(&tempty, tph ^ 1u, kWaitNs, &abort_flag)) ||
-                    !tc::wait_timed(&full[s], ph, kWaitNs, &abort_flag)) {
-                    if (lane == 0 && !abort_flag) report_fault(p.fault, kFaultTcMmaWait);
-                    abort_flag = 1;
+                if ((kb == 0 && !tc::wait_warp(&tempty, tph ^ 1u, kWaitNs, &abort_flag)) ||
+                    !tc::wait_warp(&full[s], ph, kWaitNs, &abort_flag)) {
+                    if (lane == 0) {
+                        if (!abort_flag) report_fault(p.fault, kFaultTcMmaWait);
+                        abort_flag = 1;
+                    }
                     stop = true;
                     break;
                 }
@@ -660,7 +668,7 @@ __global__ void __launch_bounds__(kThreads2, 1)
         for (int64_t t = unit; t < total; t += units, tph ^= 1u) {
             int tm, tn, z;
             decode(t, tm, tn, z);
-            if (!tc::wait_timed(&tfull, tph, 2 * kWaitNs, &abort_flag)) {
+            if (!tc::wait_warp(&tfull, tph, 2 * kWaitNs, &abort_flag)) {
                 if (!abort_flag) report_fault(p.fault, kFaultTcEpilogueWait);
                 abort_flag = 1;
                 break;

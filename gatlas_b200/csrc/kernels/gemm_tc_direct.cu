@@ -275,11 +275,13 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_direct_kernel(const __gri
             bool stop = false;
             for (int i = 0; i < nsl; ++i) {
                 const bool first = in_seg == 0;
-                if (first && !tc::wait_timed(&tempty[b], bph, kWaitNs, &abort_flag)) stop = true;
-                if (!stop && !tc::wait_timed(&full[s], ph, kWaitNs, &abort_flag)) stop = true;
+                if (first && !tc::wait_warp(&tempty[b], bph, kWaitNs, &abort_flag)) stop = true;
+                if (!stop && !tc::wait_warp(&full[s], ph, kWaitNs, &abort_flag)) stop = true;
                 if (stop) {
-                    if (!abort_flag && lane == 0) report_fault(a.fault, kFaultTcMmaWait);
-                    abort_flag = 1;
+                    if (lane == 0) {
+                        if (!abort_flag) report_fault(a.fault, kFaultTcMmaWait);
+                        abort_flag = 1;
+                    }
                     break;
                 }
                 tc::fence_after_sync();
@@ -382,7 +384,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_direct_kernel(const __gri
         bool ok = true;
         auto drain = [&]() {
             const int b = drained % kBuffers;
-            if (!tc::wait_timed(&tfull[b], (uint32_t)(drained / kBuffers) & 1u, 2 * kWaitNs, &abort_flag)) {
+            if (!tc::wait_warp(&tfull[b], (uint32_t)(drained / kBuffers) & 1u, 2 * kWaitNs, &abort_flag)) {
                 if (!abort_flag) report_fault(a.fault, kFaultTcEpilogueWait);
                 abort_flag = 1;
                 ok = false;
@@ -410,7 +412,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_direct_kernel(const __gri
             // the MMAs this stage waits for may wait for a buffer of ours
             while (ok && (int64_t)(drained + kBuffers) * seg <= i - S) drain();
             if (!ok) break;
-            if (!tc::wait_timed(&empty[s], ((uint32_t)(i / S) & 1u) ^ 1u, kWaitNs, &abort_flag)) {
+            if (!tc::wait_warp(&empty[s], ((uint32_t)(i / S) & 1u) ^ 1u, kWaitNs, &abort_flag)) {
                 if (!abort_flag) report_fault(a.fault, kFaultTcProducerWait);
                 abort_flag = 1;
                 ok = false;

@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     for (int64_t it = 0; it < items; ++it) {
         const int s = (int)(it % RS);
         const uint32_t ph = (uint32_t)(it / RS) & 1u;
-        if (!tc::wait_timed(&full[s], ph, kWaitNs, &abort_flag)) {
+        if (!tc::wait_warp(&full[s], ph, kWaitNs, &abort_flag)) {
             if (!abort_flag) report_fault(a.fault, kFaultGemvTmaWait);
             abort_flag = 1;
             break;
@@ -256,7 +256,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (int64_t b = 0; b < nboxes; ++b) {
             const int s = (int)(b % CS);
             const uint32_t ph = (uint32_t)(b / CS) & 1u;
-            if (!tc::wait_timed(&full[s], ph, kWaitNs, &abort_flag)) {
+            if (!tc::wait_warp(&full[s], ph, kWaitNs, &abort_flag)) {
                 if (!abort_flag) report_fault(a.fault, kFaultGemvTmaWait);
                 abort_flag = 1;
                 break;

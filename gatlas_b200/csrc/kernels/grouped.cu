@@ -376,9 +376,13 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_kernel(Params p) {
     const bool leader = rank == 0;
     const int unit = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
     const int t_begin = p.cta_start[unit], t_end = p.cta_start[unit + 1];
-    auto wait = [&](uint64_t *bar, uint32_t parity, uint64_t limit) {
+    auto wait_lane = [&](uint64_t *bar, uint32_t parity, uint64_t limit) {
         return PAIR ? tc::wait_timed_cluster(bar, parity, limit, &abort_flag)
                     : tc::wait_timed(bar, parity, limit, &abort_flag);
+    };
+    auto wait_warp = [&](uint64_t *bar, uint32_t parity, uint64_t limit) {
+        return PAIR ? tc::wait_warp_cluster(bar, parity, limit, &abort_flag)
+                    : tc::wait_warp(bar, parity, limit, &abort_flag);
     };
 
     if (threadIdx.x == 0) {
@@ -435,9 +439,11 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_kernel(Params p) {
             const int64_t a_off = (PAIR && rank == 1 && cur.rows > BM) ? (int64_t)cur.kt * kATileBytes : 0;
             const int64_t b_off = PAIR ? (int64_t)rank * b_bytes : 0;
             for (int kb = 0; kb < cur.kt; ++kb, ++ring) {
-                if (!wait(&empty[s], ph ^ 1u, kWaitNs)) {
-                    if (lane == 0 && !abort_flag) report_fault(p.fault, kFaultTcProducerWait);
-                    abort_flag = 1;
+                if (!wait_warp(&empty[s], ph ^ 1u, kWaitNs)) {
+                    if (lane == 0) {
+                        if (!abort_flag) report_fault(p.fault, kFaultTcProducerWait);
+                        abort_flag = 1;
+                    }
                     stop = true;
                     break;
                 }
@@ -468,7 +474,7 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_kernel(Params p) {
                 const int kt = p.tiles[t].kt;
                 for (int kb = 0; kb < kt; ++kb, ++ring) {
                     const int s = ring % S;
-                    if (!wait(&full[s], (uint32_t)(ring / S) & 1u, kWaitNs)) {
+                    if (!wait_lane(&full[s], (uint32_t)(ring / S) & 1u, kWaitNs)) {
                         if (!abort_flag) report_fault(p.fault, kFaultTcProducerWait);
                         abort_flag = 1;
                         stop = true;
@@ -503,10 +509,12 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_kernel(Params p) {
                     const int b = seg & 1;
                     const bool seg_first = in_seg == 0;
                     const bool seg_last = ++in_seg == p.seg_kblocks || kb == kt - 1;
-                    if ((seg_first && !wait(&tempty[b], ((uint32_t)(seg >> 1) & 1u) ^ 1u, kWaitNs)) ||
-                        !wait(&full[s], ph, kWaitNs)) {
-                        if (lane == 0 && !abort_flag) report_fault(p.fault, kFaultTcMmaWait);
-                        abort_flag = 1;
+                    if ((seg_first && !wait_warp(&tempty[b], ((uint32_t)(seg >> 1) & 1u) ^ 1u, kWaitNs)) ||
+                        !wait_warp(&full[s], ph, kWaitNs)) {
+                        if (lane == 0) {
+                            if (!abort_flag) report_fault(p.fault, kFaultTcMmaWait);
+                            abort_flag = 1;
+                        }
                         stop = true;
                         break;
                     }
@@ -595,8 +603,7 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_kernel(Params p) {
             }
             for (int sg = 0; sg < nseg; ++sg, ++seg) {
                 const int b = seg & 1;
-                // the warp leaves together: it meets again below
-                if (!__all_sync(0xffffffffu, wait(&tfull[b], (uint32_t)(seg >> 1) & 1u, 2 * kWaitNs))) {
+                if (!wait_warp(&tfull[b], (uint32_t)(seg >> 1) & 1u, 2 * kWaitNs)) {
                     if (!abort_flag) report_fault(p.fault, kFaultTcEpilogueWait);
                     abort_flag = 1;
                     ok = false;

@@ -25,8 +25,8 @@ __device__ __forceinline__ uint64_t globaltimer() {
     return t;
 }
 
-// mbarrier wait bounded in wall time (ns).  Returns false on timeout or when
-// *abort becomes non-zero.
+// mbarrier wait of one thread, bounded in wall time (ns).  Returns false on
+// timeout or when *abort becomes non-zero.
 __device__ __forceinline__ bool wait_timed(uint64_t *bar, uint32_t parity, uint64_t limit_ns,
                                            volatile int *abort) {
     if (mbar_try_wait(bar, parity)) return true;
@@ -36,6 +36,15 @@ __device__ __forceinline__ bool wait_timed(uint64_t *bar, uint32_t parity, uint6
         if (abort && *abort) return false;
         if (globaltimer() - t0 > limit_ns) return false;
     }
+}
+
+// The same for a whole converged warp.  Each lane polls by itself and may give
+// up by itself (its own clock, the abort flag), so the lanes agree before one
+// of them acts on the answer: false where any lane gave up.  Without the vote
+// some lanes would leave while others went on to warp-wide instructions
+// (elect.sync, TMEM loads) that then never complete.
+__device__ __forceinline__ bool wait_warp(uint64_t *bar, uint32_t parity, uint64_t limit_ns, volatile int *abort) {
+    return __all_sync(0xffffffffu, wait_timed(bar, parity, limit_ns, abort));
 }
 
 enum Swizzle : uint32_t { kSwizzleNone = 0, kSwizzle128B = 2, kSwizzle64B = 4, kSwizzle32B = 6 };
@@ -205,6 +214,11 @@ __device__ __forceinline__ bool wait_timed_cluster(uint64_t *bar, uint32_t parit
         if (abort && *abort) return false;
         if (globaltimer() - t0 > limit_ns) return false;
     }
+}
+
+__device__ __forceinline__ bool wait_warp_cluster(uint64_t *bar, uint32_t parity, uint64_t limit_ns,
+                                                  volatile int *abort) {
+    return __all_sync(0xffffffffu, wait_timed_cluster(bar, parity, limit_ns, abort));
 }
 
 // Arrive on an mbarrier of another CTA of the cluster (shared::cluster address).

@@ -460,6 +460,13 @@ int gatlas_device_faults(int *flags, int clear);
  * No reference counterpart. */
 int gatlas_selftest_bounded_wait(int64_t limit_ns, int arrive, int *completed, void *stream);
 
+/* The same for a whole warp, whose lanes must leave a wait together: half of
+ * them give up before the phase completes (after limit_ns / 2), the others
+ * would not.  *completed is the number of lanes told that it did (0), *elected
+ * the number elected afterwards by a warp-wide instruction (1); bit 6 of the
+ * fault word is set.  No reference counterpart. */
+int gatlas_selftest_warp_wait(int64_t limit_ns, int *completed, int *elected, void *stream);
+
 #ifdef __cplusplus
 }
 #endif
