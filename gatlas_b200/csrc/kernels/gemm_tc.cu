@@ -1372,7 +1372,7 @@ static int launch_wide(const Geometry &g, const Plan &pl, const WsPtrs &w, Param
 
 template <int MODE>
 static int launch_tc(const Geometry &g, const Plan &pl, const WsPtrs &w, float *C, double alpha, double beta,
-                     int gemm, int seg_kblocks, cudaStream_t stream) {
+                     int gemm, uint32_t extra, cudaStream_t stream) {
     using L = Layout<MODE>;
     const int64_t pair_tiles = ((g.M + 2 * BM - 1) / (2 * BM)) * ((g.N + BN - 1) / BN) * g.batch;
     const bool pair = g.M > BM && (g_tc_pair == 2 || (g_tc_pair == 1 && (MODE == 1 || MODE == 2 ||
@@ -1402,7 +1402,7 @@ static int launch_tc(const Geometry &g, const Plan &pl, const WsPtrs &w, float *
     p.ldc = g.ldc;
     p.stride_c = g.stride_c;
     p.kblocks = (int)((pl.Kp + L::BK - 1) / L::BK);
-    p.seg_kblocks = seg_kblocks > 0 ? seg_kblocks : default_seg_kblocks(MODE);
+    p.seg_kblocks = promotion_interval(extra, MODE, p.kblocks);
     p.alpha = (float)alpha;
     p.beta = (float)beta;
     p.gemm = gemm;
@@ -1489,10 +1489,10 @@ int tc_run(const gatlas_matmul_desc *d, const Geometry &g, const void *ws, size_
     if (g.K == 0) return set_error(GATLAS_ERR_INVALID, "matmul: K == 0 has no prepared operands");
     const WsPtrs w = ws_ptrs(pl, const_cast<void *>(ws));
     switch (pl.mode) {
-        case 0: return launch_tc<0>(g, pl, w, C, d->alpha, d->beta, d->gemm, (int)d->extra, stream);
-        case 1: return launch_tc<1>(g, pl, w, C, d->alpha, d->beta, d->gemm, (int)d->extra, stream);
-        case 2: return launch_tc<2>(g, pl, w, C, d->alpha, d->beta, d->gemm, (int)d->extra, stream);
-        default: return launch_tc<3>(g, pl, w, C, d->alpha, d->beta, d->gemm, (int)d->extra, stream);
+        case 0: return launch_tc<0>(g, pl, w, C, d->alpha, d->beta, d->gemm, d->extra, stream);
+        case 1: return launch_tc<1>(g, pl, w, C, d->alpha, d->beta, d->gemm, d->extra, stream);
+        case 2: return launch_tc<2>(g, pl, w, C, d->alpha, d->beta, d->gemm, d->extra, stream);
+        default: return launch_tc<3>(g, pl, w, C, d->alpha, d->beta, d->gemm, d->extra, stream);
     }
 }
 
@@ -1550,10 +1550,10 @@ static int run_rows(const gatlas_matmul_desc *d, const Plan &pl, const Geometry 
     }
     float *Cb = C + r0 * g.ldc;
     switch (pl.mode) {
-        case 0: return launch_tc<0>(gb, pb, wb, Cb, d->alpha, d->beta, d->gemm, (int)d->extra, s);
-        case 1: return launch_tc<1>(gb, pb, wb, Cb, d->alpha, d->beta, d->gemm, (int)d->extra, s);
-        case 2: return launch_tc<2>(gb, pb, wb, Cb, d->alpha, d->beta, d->gemm, (int)d->extra, s);
-        default: return launch_tc<3>(gb, pb, wb, Cb, d->alpha, d->beta, d->gemm, (int)d->extra, s);
+        case 0: return launch_tc<0>(gb, pb, wb, Cb, d->alpha, d->beta, d->gemm, d->extra, s);
+        case 1: return launch_tc<1>(gb, pb, wb, Cb, d->alpha, d->beta, d->gemm, d->extra, s);
+        case 2: return launch_tc<2>(gb, pb, wb, Cb, d->alpha, d->beta, d->gemm, d->extra, s);
+        default: return launch_tc<3>(gb, pb, wb, Cb, d->alpha, d->beta, d->gemm, d->extra, s);
     }
 }
 

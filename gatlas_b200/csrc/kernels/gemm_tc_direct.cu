@@ -590,8 +590,9 @@ int matmul_direct(const gatlas_matmul_desc *d, const Geometry &g, int bn, const 
     a.C = C;
     a.M = g.M, a.N = g.N, a.K = g.K, a.ldc = g.ldc, a.stride_c = g.stride_c;
     a.nslices = (int)((g.K + kSlice - 1) / kSlice);
-    const int interval = d->extra > 0 ? (int)d->extra : default_seg_kblocks(mode);
-    a.seg = mode == 2 ? interval / 2 : interval;
+    // (split6 counts slices of 32; its interval here is even)
+    a.seg = mode == 2 ? promotion_interval(d->extra, mode, 2 * a.nslices) / 2
+                      : promotion_interval(d->extra, mode, a.nslices);
     // the two-pass path stages split6 in slices of 32: half a slice of steps where the second half is empty
     a.last_ksteps = mode == 2 && g.K - (int64_t)(a.nslices - 1) * kSlice <= 32 ? 2 : kSlice / 16;
     a.alpha = (float)d->alpha, a.beta = (float)d->beta, a.gemm = d->gemm;

@@ -30,6 +30,13 @@ constexpr int kSegAll = 1 << 30;
 __host__ __device__ constexpr int default_seg_kblocks(int mode) {
     return mode == 0 ? kSegAll : mode == 3 ? 16 : 4;
 }
+// A call's promotion interval: the descriptor's extra as a signed count (0 and
+// below: the mode's default), and never more than the `slices` there are, so
+// that counts of segments are at least 1 and stay within 32 bits.
+inline int promotion_interval(uint32_t extra, int mode, int slices) {
+    const int asked = (int)extra > 0 ? (int)extra : default_seg_kblocks(mode);
+    return asked < slices ? asked : (slices > 0 ? slices : 1);
+}
 // FP8: most 128-deep blocks per tile (K <= 131072).
 constexpr int kMaxFp8Blocks = 1024;
 
