@@ -13,6 +13,7 @@
 #include <string.h>
 
 #include "../common.cuh"
+#include "../tcgen05.cuh"
 
 namespace gatlas {
 namespace gvc {
@@ -136,7 +137,7 @@ __global__ void __launch_bounds__(kThreads) gemv_cols_cluster_kernel(Args a) {
         sums[threadIdx.x] = t;
     }
     const unsigned nseg = gridDim.y;
-    if (nseg > 1) asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (nseg > 1) tc::cluster_sync();
     else __syncthreads();
     const size_t col = col0 + threadIdx.x;
     if (seg == 0 && threadIdx.x < W && col < a.M) {
@@ -154,7 +155,7 @@ __global__ void __launch_bounds__(kThreads) gemv_cols_cluster_kernel(Args a) {
         *y = t;
     }
     // no CTA leaves while the first may still read its sums
-    if (nseg > 1) asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (nseg > 1) tc::cluster_sync();
 }
 
 }  // namespace gvc

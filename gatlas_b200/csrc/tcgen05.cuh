@@ -191,8 +191,10 @@ __device__ __forceinline__ uint32_t mapa_shared(uint32_t addr, uint32_t rank) {
     return r;
 }
 
-// Whole-cluster execution barrier (every thread of both CTAs).
+// Whole-cluster execution barrier (every thread of every CTA).  The aligned
+// forms need converged warps, whatever the code before them branched on.
 __device__ __forceinline__ void cluster_sync() {
+    __syncwarp();
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 

@@ -43,3 +43,14 @@ def test_single_lane_waits_stand_under_a_single_lane():
             assert any(re.search(r"lane == 0|threadIdx\.x == 0|auto wait_lane", a) for a in around), \
                 f"{os.path.basename(path)}:{i + 1}: {line.strip()}"
     assert calls > 0
+
+
+def test_aligned_cluster_barriers_stand_behind_a_converged_warp():
+    """barrier.cluster's aligned forms appear once, in the helper that
+    converges the warp first."""
+    uses = []
+    for path in sorted(glob.glob(os.path.join(os.path.dirname(KERNELS), "**", "*.cu*"), recursive=True)):
+        text = open(path).read()
+        uses += [text[:m.start()] for m in re.finditer(r"barrier\.cluster\.arrive[a-z.]*\.aligned", text)]
+    assert len(uses) == 1
+    assert re.search(r"void cluster_sync\(\) \{\n    __syncwarp\(\);\n    asm volatile\(\"$", uses[0])
