@@ -126,10 +126,10 @@ __global__ void __launch_bounds__(kThreads, 1)
     for (int64_t it = 0; it < items; ++it) {
         const int s = (int)(it % RS);
         const uint32_t ph = (uint32_t)(it / RS) & 1u;
-        if (!tc::wait_warp(&full[s], ph, kWaitNs, &abort_flag)) {
+        if (!tc::wait_or_exit(&full[s], ph, kWaitNs, &abort_flag)) {
             if (!abort_flag) report_fault(a.fault, kFaultGemvTmaWait);
             abort_flag = 1;
-            break;
+            return;
         }
         const int64_t c = it % nchunks;
         const int64_t c0 = c * RC;
@@ -256,10 +256,10 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (int64_t b = 0; b < nboxes; ++b) {
             const int s = (int)(b % CS);
             const uint32_t ph = (uint32_t)(b / CS) & 1u;
-            if (!tc::wait_warp(&full[s], ph, kWaitNs, &abort_flag)) {
+            if (!tc::wait_or_exit(&full[s], ph, kWaitNs, &abort_flag)) {
                 if (!abort_flag) report_fault(a.fault, kFaultGemvTmaWait);
                 abort_flag = 1;
-                break;
+                return;
             }
             const int64_t r0 = j0 + b * CR;
             const int64_t rows = (j1 - r0 < CR) ? j1 - r0 : CR;

@@ -47,6 +47,14 @@ __device__ __forceinline__ bool wait_warp(uint64_t *bar, uint32_t parity, uint64
     return __all_sync(0xffffffffu, wait_timed(bar, parity, limit_ns, abort));
 }
 
+// The same where each lane that gives up returns from the kernel: the syncs,
+// barriers and shuffles of the others wait only for threads that have not exited.
+// (For the TMA GEMV kernels, whose warps wait once per 2 to 4 KiB: a vote after each
+// wait cost them 3 %.)
+__device__ __forceinline__ bool wait_or_exit(uint64_t *bar, uint32_t parity, uint64_t limit_ns, volatile int *abort) {
+    return wait_timed(bar, parity, limit_ns, abort);
+}
+
 enum Swizzle : uint32_t { kSwizzleNone = 0, kSwizzle128B = 2, kSwizzle64B = 4, kSwizzle32B = 6 };
 
 // K-major operand descriptor: 8-row core-matrix groups `sbo_bytes` apart,
