@@ -28,6 +28,8 @@
 // 17.2 us, row-major 45.6 -> 17.6; 1024 x 32767 207 -> 32; 1024^2 column-major
 // 12.5 -> 4.3, row-major 4.5 -> 3.3; 32768 x 1024 column-major 36.5 -> 22.1.
 #include <algorithm>
+#include <atomic>
+#include <cmath>
 
 #include "../common.cuh"
 #include "../device_state.cuh"
@@ -438,101 +440,163 @@ static bool gemv_vec_ok(const gatlas_matvec_desc *d, const T *A, const T *x) {
 }
 
 // Column-major products whose segments fit one cluster (gemv_cols.cuh).
-// nseg == 0: the general kernel, with partial sums in a workspace, serves it:
-// too few column blocks for clusters of 8 to fill the GPU, or doubles off the
-// 16-byte grid (26 us at 2479 x 5702 against 33).
+constexpr int kMaxSegments = 8;  // CTAs of a portable cluster
+struct ClusterKernel {
+    const void *fn;
+    size_t width;                                     // columns per block
+    bool even;                                        // segments dealt evenly to SMs (see cluster_plan)
+    std::atomic<int> resident[64][kMaxSegments + 1];  // per device and cluster size, 0: not asked yet
+};
 struct ClusterPlan {
-    int variant, nseg;
-    size_t width;
+    const ClusterKernel *kernel;
+    int nseg;  // 0: the general kernel, with partial sums in a workspace
 };
 
-template <typename T>
-static ClusterPlan cluster_plan(const gatlas_matvec_desc *d, bool vec_ok) {
-    ClusterPlan c{0, 0, 0};
-    const size_t batch = d->batch ? d->batch : 1;
-    if (d->n == 0 || (sizeof(T) == 8 && !vec_ok)) return c;
-    const size_t sms = (size_t)sm_count();
-    const auto blocks_of = [&](size_t width) { return (d->m + width - 1) / width * batch; };
-    // CTAs that a cluster launch is sure to have resident, in tenths of an SM:
-    // with more, a second wave of clusters doubles the time.  Fewer than fit one
-    // by one, since a cluster needs its CTAs in one place (3456 x 22652 floats,
-    // 54 blocks: 64 us with 8 segments, 50 with 7).
-    size_t tenths = 40;
-    if (sizeof(T) == 4 && vec_ok) {
-        // 64 columns, 16 rows in flight, wherever clusters of them fill the GPU and
-        // fit it (1716 x 19132: 27 us, with 32 columns 34, with 128 36; 16384^2 155,
-        // 184 and 160; 6772 x 3024 13, 16 and 14); 32 columns where there are too
-        // few blocks of 64, or so many that clusters of two no longer fit but single
-        // CTAs of 32 columns do (14000 x 6000: 53 us, 64 columns 56); 128 beyond
-        // (30000 x 4000: 78 us, 64 columns 90)
-        const size_t fit = sms * 27 / 10;
-        const bool pairs = blocks_of(64) * 2 <= fit, singles = blocks_of(32) <= sms * 3;
-        if (blocks_of(64) * 32 < sms * 5 || (!pairs && singles)) c.variant = 0, c.width = 32;
-        else if (blocks_of(64) <= fit) c.variant = 2, c.width = 64;
-        else c.variant = 1, c.width = 128;
-        if (c.variant != 1) tenths = 27;
-    } else if (sizeof(T) == 4) {
-        // off the 16-byte grid: 32 columns with more rows in flight up to 2048
-        // columns, 64 beyond (2047 x 20001: 34 us and 38; 3001 x 7013 19 and 15)
-        const bool narrow = d->m <= 2048;
-        c.variant = narrow ? 0 : 1, c.width = narrow ? 32 : 64;
-        tenths = narrow ? 30 : 35;  // (5001 x 14003: 67 us with 40, 54 with 35)
-    } else {
-        // doubles: 32 columns up to 4096, and where blocks of 64 are too many for
-        // clusters of two but leave SMs with two CTAs beside others with three
-        // (26804 x 3376: 110 us with 32, 126 with 64; 30000 x 2000 98 and 82, 8700 x
-        // 1588 23 and 22, 4720 x 9744 62 and 60)
-        const bool narrow = d->m <= 4096 || (blocks_of(64) > 2 * sms && blocks_of(64) <= 3 * sms);
-        c.variant = narrow ? 0 : 1, c.width = narrow ? 32 : 64;
-    }
-    const size_t blocks = blocks_of(c.width);
-    if (blocks * 8 < sms || blocks / batch > 0x7fffffffu) return c;
-    // clusters of up to 8 CTAs, as many in all as are resident, each of 64 rows at
-    // least (5596 x 19076 doubles 196 us with 704 CTAs, 135 with 528)
-    const size_t resident = sms * tenths / 10;
-    int nseg = 8;
-    while (nseg > 1 && (blocks * (size_t)nseg > resident || (size_t)nseg * 64 > d->n)) --nseg;
-    // long segments on SMs with two and three CTAs: the general kernel's finer
-    // segments even out (doubles, 1450 x 31575: 79 us, 67 there; 1176 x 12000 31 and
-    // 28; 1176 x 8192 21 both)
-    if (sizeof(T) == 8 && nseg == 8 && blocks * 8 < 3 * sms && d->n >= 10240) return c;
-    c.nseg = nseg;
-    return c;
+static cudaLaunchConfig_t cluster_config(dim3 grid, int nseg, cudaLaunchAttribute *attr, cudaStream_t stream) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(gvc::kThreads, 1, 1);
+    cfg.stream = stream;
+    attr->id = cudaLaunchAttributeClusterDimension;
+    attr->val.clusterDim.x = 1;
+    attr->val.clusterDim.y = (unsigned)nseg;
+    attr->val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cfg;
 }
 
+// Clusters of nseg CTAs that the current device (dev) holds at once.  Fewer than its
+// CTAs over nseg, since a cluster needs its CTAs in one place: three CTAs per SM
+// make 222 clusters of 2, but 104 of 4 and 48 of 8.  With one cluster more a second
+// wave nearly doubles the time (3396 x 27644 doubles: 111 us at 0.92 of what
+// fits, 149 at 1.10).
+static size_t clusters_resident(ClusterKernel &k, int dev, int nseg) {
+    std::atomic<int> &known = k.resident[dev & 63][nseg];
+    int n = known.load(std::memory_order_relaxed);
+    if (n == 0) {
+        cudaLaunchAttribute attr;
+        const cudaLaunchConfig_t cfg = cluster_config(dim3(1, (unsigned)nseg, 1), nseg, &attr, nullptr);
+        if (cudaOccupancyMaxActiveClusters(&n, k.fn, &cfg) != cudaSuccess || n <= 0) {
+            cudaGetLastError();
+            n = std::max(1, sm_count() * 2 / nseg);
+        }
+        known.store(n, std::memory_order_relaxed);
+    }
+    return (size_t)n;
+}
+
+// The kernel by columns (times instances), then as many segments as fit at once,
+// of 256 rows at least (2602 x 517 floats 6.2 us, 7.2 in 8 segments), 512 of up to 64
+// floats where the blocks alone fill the SMs (13676 x 992 8.2 us, 10.2 in two).
 template <typename T>
-static int launch_cluster(const GemvArgs &g, const ClusterPlan &cp, bool vec_ok, size_t batch, cudaStream_t stream) {
+static ClusterPlan cluster_plan(const gatlas_matvec_desc *d, bool vec_ok) {
+    constexpr int V = 16 / (int)sizeof(T);
+    const ClusterPlan general{nullptr, 0};
+    const size_t batch = d->batch ? d->batch : 1, sms = (size_t)sm_count();
+    const auto blocks_of = [&](size_t width) { return (d->m + width - 1) / width * batch; };
+    if (d->n == 0 || blocks_of(32) * 8 < sms) return general;  // too few blocks for clusters of 8
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const auto segments = [&](ClusterKernel &k) {
+        const size_t rows = sizeof(T) == 4 && k.width <= 64 && blocks_of(k.width) >= sms ? 512 : 256;
+        int s = kMaxSegments;
+        while (s > 1 && ((size_t)s * rows > d->n || blocks_of(k.width) > clusters_resident(k, dev, s))) --s;
+        return s;
+    };
+    // blocks over what fits at once, and that over whole waves
+    const auto fill = [&](ClusterKernel &k, int s) { return (double)blocks_of(k.width) / (double)clusters_resident(k, dev, s); };
+    const auto wave_share = [](double f) { return f / std::ceil(f); };
+    ClusterKernel *k;
+    if constexpr (sizeof(T) == 4) {
+        static ClusterKernel vec[] = {{(const void *)gvc::gemv_cols_cluster_kernel<T, true, 8, V, 16, 0, 0>, 32, false, {}},
+                                      {(const void *)gvc::gemv_cols_cluster_kernel<T, true, 16, V, 16, 0, 0>, 64, false, {}},
+                                      {(const void *)gvc::gemv_cols_cluster_kernel<T, true, 32, V, 8, 0, 0>, 128, false, {}}};
+        static ClusterKernel one[] = {{(const void *)gvc::gemv_cols_cluster_kernel<T, false, 16, 2, 16, 0, 0>, 32, true, {}},
+                                      {(const void *)gvc::gemv_cols_cluster_kernel<T, false, 32, 2, 16, 0, 0>, 64, false, {}},
+                                      {(const void *)gvc::gemv_cols_cluster_kernel<T, false, 16, 4, 8, 1, 0>, 64, false, {}},
+                                      {(const void *)gemv_cols_kernel<T, 1, 4>, 32, false, {}}};
+        if (vec_ok) {
+            // 32 columns until clusters of 8 on 64 columns fill half the GPU (868 x
+            // 10563 9.1 us against 10.2, 1116 x 56216 49 and 53; 1524 x 1905 8.3 and
+            // 6.3), then 64 until clusters of two just fit (12000 x 10000 72 us, 128
+            // columns 74; 13604 x 14780 123 and 118; 30000 x 4000 90 and 74), or while
+            // they fit where columns are short (17236 x 452 6.2 and 8.2).  Long columns
+            // again where single CTAs of 128 are under 2/3 of what fits or over it
+            // (40000 x 6000 147 and 157, 100000 x 2000 120 and 132; 60000 x 500 25 and
+            // 22); just over it the general kernel (80000 x 1000 48 us, 64 columns 52).
+            const bool brief = d->n < 1024;
+            const double f128 = fill(vec[2], 1);
+            if (f128 > 1 && f128 <= 1.25) return general;
+            if (blocks_of(64) * 2 < clusters_resident(vec[1], dev, 8)) k = &vec[0];
+            else if (fill(vec[1], 2) <= 0.9 || (brief && fill(vec[1], 1) <= 1)) k = &vec[1];
+            else k = &vec[brief || fill(vec[2], 2) <= 1 || (f128 * 3 > 2 && f128 <= 1) ? 2 : 1];
+        } else if (blocks_of(32) * 2 <= sms) {
+            // off the 16-byte grid: 32 columns up to half a block per SM (1001 x 30001
+            // 29 us, 64 columns 45; 2203 x 30011 52 and 54; 3301 x 20003 52 and 50)
+            k = &one[0];
+        } else {
+            // 64 columns: 16 rows in flight, or 8 where columns are short (3001 x 7013 17.3
+            // us and 16.5, 9001 x 3001 21.4 and 20.6; 5001 x 14003 50 and 52) or more CTAs
+            // then fill the GPU better (15001 x 9001 110 and 95)
+            const int s1 = segments(one[1]), s2 = segments(one[2]);
+            k = &one[d->n < 8192 || fill(one[2], s2) > fill(one[1], s1) + 0.1 ? 2 : 1];
+            // from about 20800 columns the general kernel's many small CTAs are faster
+            // (22003 x 3001 46 us and 49) unless their last wave is nearly empty (30001 x
+            // 4001 113 and 83)
+            if (blocks_of(64) * 10 > sms * 22) {
+                k = &one[2];
+                if (wave_share(fill(one[3], 1)) * 1.1 >= wave_share(fill(one[2], 1))) return general;
+            }
+        }
+    } else {
+        static ClusterKernel vec[] = {{(const void *)gvc::gemv_cols_cluster_kernel<T, true, 16, V, 8, 2, 5>, 32, false, {}},
+                                      {(const void *)gvc::gemv_cols_cluster_kernel<T, true, 32, V, 8, 2, 5>, 64, false, {}},
+                                      {(const void *)gvc::gemv_cols_cluster_kernel<T, true, 16, V, 8, 2, 6>, 32, false, {}}};
+        // off the 16-byte grid the general kernel is faster (2479 x 5702: 26 us against 33)
+        if (!vec_ok) return general;
+        // 32 columns until clusters of 8 on 64 fill three quarters of the GPU (3872 x
+        // 16820 79 us, 64 columns 82; 6732 x 5348 49 and 47), while they fit where
+        // columns are short, and again where blocks of 64 no longer fit (44728 x 4940 255
+        // and 251; 59288 x 2516 179 and 196) unless the last wave is nearly empty (50002
+        // x 5002 331, general kernel 293; 56388 x 3720, 0.4 full, 252 and 269)
+        const double f32 = fill(vec[0], 1), f64 = fill(vec[1], 1);
+        if (f64 > 1 && f32 - std::floor(f32) < 0.33) return general;
+        if (f32 > 1 && fill(vec[2], 1) <= 1) k = &vec[2];
+        else k = &vec[blocks_of(64) * 4 > clusters_resident(vec[1], dev, 8) * 3 && f64 <= 1 && (d->n >= 512 || f32 > 1) ? 1 : 0];
+    }
+    const size_t blocks = blocks_of(k->width);
+    if (blocks * 8 < sms || blocks / batch > 0x7fffffffu) return general;
+    int nseg = segments(*k);
+    // The narrow kernel off the 16-byte grid is bound by the SM with the most rows:
+    // whole CTAs per SM (3 % fewer SMs, since clusters do not pack them all) over the
+    // segment count (1617 x 13049, 51 blocks: 18.6 us with 5 segments, 20.6 with 7;
+    // 1411 x 40003, 45: 45 with 6, 49 with 8).
+    if (k->even) {
+        const size_t even_sms = sms * 97 / 100;
+        const auto load = [&](int s) { return (double)((blocks * s + even_sms - 1) / even_sms) / s; };
+        for (int s = nseg - 1; s >= 1; --s)
+            if (load(s) < load(nseg)) nseg = s;
+    }
+    // few columns and long rows of doubles: the general kernel cuts the rows finer,
+    // as fast (1450 x 31575: 66 us both, 1392 x 10148 25 and 27) and with shorter sums
+    if (sizeof(T) == 8 && nseg == 8 && blocks * 8 < 3 * sms && d->n >= 9216) return general;
+    return {k, nseg};
+}
+
+static int launch_cluster(const GemvArgs &g, const ClusterPlan &cp, size_t batch, cudaStream_t stream) {
     gvc::Args a;
     a.A = g.A, a.x = g.x, a.y = g.y;
     a.M = g.M, a.N = g.N, a.lda = g.lda;
     a.stride_a = g.stride_a, a.stride_x = g.stride_x, a.stride_y = g.stride_y;
     a.alpha = g.alpha, a.beta = g.beta, a.gemv = g.gemv;
     a.seg_len = (g.N + cp.nseg - 1) / cp.nseg;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)((g.M + cp.width - 1) / cp.width), (unsigned)cp.nseg, (unsigned)batch);
-    cfg.blockDim = dim3(gvc::kThreads, 1, 1);
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 1;
-    attr[0].val.clusterDim.y = (unsigned)cp.nseg;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    constexpr int V = 16 / (int)sizeof(T);
-    cudaError_t e;
-    if constexpr (sizeof(T) == 4) {
-        if (vec_ok)
-            e = cp.variant == 0   ? cudaLaunchKernelEx(&cfg, gvc::gemv_cols_cluster_kernel<T, true, 8, V, 16>, a)
-                : cp.variant == 1 ? cudaLaunchKernelEx(&cfg, gvc::gemv_cols_cluster_kernel<T, true, 32, V, 8>, a)
-                                  : cudaLaunchKernelEx(&cfg, gvc::gemv_cols_cluster_kernel<T, true, 16, V, 16>, a);
-        else
-            e = cp.variant == 0 ? cudaLaunchKernelEx(&cfg, gvc::gemv_cols_cluster_kernel<T, false, 16, 2, 16>, a)
-                                : cudaLaunchKernelEx(&cfg, gvc::gemv_cols_cluster_kernel<T, false, 16, 4, 8>, a);
-    } else {
-        e = cp.variant == 0 ? cudaLaunchKernelEx(&cfg, gvc::gemv_cols_cluster_kernel<T, true, 16, V, 8>, a)
-                            : cudaLaunchKernelEx(&cfg, gvc::gemv_cols_cluster_kernel<T, true, 32, V, 8>, a);
-    }
+    const size_t width = cp.kernel->width;
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t cfg = cluster_config(
+        dim3((unsigned)((g.M + width - 1) / width), (unsigned)cp.nseg, (unsigned)batch), cp.nseg, &attr, stream);
+    void *args[] = {&a};
+    const cudaError_t e = cudaLaunchKernelExC(&cfg, cp.kernel->fn, args);
     if (e != cudaSuccess) return set_error(GATLAS_ERR_CUDA, "gemv_cols_cluster_kernel: %s", cudaGetErrorString(e));
     return check_launch("gemv_cols_cluster_kernel");
 }
@@ -634,7 +698,7 @@ static int matvec_launch(const gatlas_matvec_desc *d, const T *A, const T *x, T 
             return set_error(GATLAS_ERR_INVALID, "matvec: workspace %zu < %zu bytes", ws_bytes, need);
         if (ws && !aligned_to(ws, 256)) return set_error(GATLAS_ERR_INVALID, "matvec: workspace must be 256-byte aligned");
     }
-    if (const ClusterPlan cp = cluster_plan<T>(d, vec_ok); cp.nseg) return launch_cluster<T>(a, cp, vec_ok, batch, stream);
+    if (const ClusterPlan cp = cluster_plan<T>(d, vec_ok); cp.nseg) return launch_cluster(a, cp, batch, stream);
     if (pl.nseg > 1) {
         const size_t need = pl.part_bytes + pl.counter_bytes;
         if (!ws) {

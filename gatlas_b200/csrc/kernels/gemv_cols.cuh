@@ -8,6 +8,17 @@
 // block's segments, one CTA of a cluster each, are added in segment order by
 // the first CTA over distributed shared memory: no partial sums in global
 // memory, no arrival counters to clear and no second launch.
+//
+// Rounding: floats are summed U rows from zero, then added to the column's
+// total, doubles into two accumulators (floats off the 16-byte grid with 8 rows
+// in flight need neither), and a block's 8 warps add up in pairs, so that the
+// sums are no longer than the general kernel's, whose 4 CTAs per SM cut the rows
+// finer (one chain per lane: error against 64 bits at 16384^2 floats 1.56 times
+// the general kernel's, at 20000 x 6000 1.3; now half).
+//
+// How many loads the compiler keeps in flight follows from what else holds
+// registers, hence an instantiation's accumulators and CTAs per SM: doubles with
+// two accumulators 116 us at 3396 x 27644, with one 128, with sums from zero 146.
 #pragma once
 
 #include <string.h>
@@ -60,9 +71,11 @@ __device__ __forceinline__ void load_one(const double *p, double &v) {
     asm volatile("ld.global.cs.f64 %0, [%1];" : "=d"(v) : "l"(p));
 }
 
-// T; VEC: 16-byte loads (CPL = 16 / sizeof(T)); LPR lanes per row; U row groups in flight
-template <typename T, bool VEC, int LPR, int CPL, int U>
-__global__ void __launch_bounds__(kThreads) gemv_cols_cluster_kernel(Args a) {
+// T; VEC: 16-byte loads (CPL = 16 / sizeof(T)); LPR lanes per row; U row groups in
+// flight; SETS accumulators per column, rows dealt out among them, or 0: one, added
+// to the column's total after every U rows; MINB CTAs per SM asked for (0: none)
+template <typename T, bool VEC, int LPR, int CPL, int U, int SETS, int MINB>
+__global__ void __launch_bounds__(kThreads, MINB) gemv_cols_cluster_kernel(Args a) {
     constexpr int W = LPR * CPL, RPW = 32 / LPR;  // columns per block, rows per warp and group
     __shared__ T red[kWarps][W];
     __shared__ T sums[W];
@@ -81,9 +94,23 @@ __global__ void __launch_bounds__(kThreads) gemv_cols_cluster_kernel(Args a) {
 #pragma unroll
     for (int c = 0; c < CPL; ++c) off[c] = VEC ? min(col0 + lc * CPL, a.M - CPL) : min(col0 + column(c), a.M - 1);
 
-    T acc[CPL];
+    constexpr int NS = SETS ? SETS : 1;
+    T acc[CPL], part[NS][CPL];
 #pragma unroll
-    for (int c = 0; c < CPL; ++c) acc[c] = T(0);
+    for (int c = 0; c < CPL; ++c) {
+        acc[c] = T(0);
+#pragma unroll
+        for (int s = 0; s < NS; ++s) part[s][c] = T(0);
+    }
+    auto total = [&]() {  // the sets into the column's total
+#pragma unroll
+        for (int c = 0; c < CPL; ++c)
+#pragma unroll
+            for (int s = 0; s < NS; ++s) {
+                acc[c] += part[s][c];
+                part[s][c] = T(0);
+            }
+    };
     constexpr int STEP = kWarps * RPW;  // rows per group of all warps
     size_t j = j0 + (size_t)w * RPW + lr;
     auto load = [&](const T *row, T (&v)[CPL]) {
@@ -104,7 +131,8 @@ __global__ void __launch_bounds__(kThreads) gemv_cols_cluster_kernel(Args a) {
 #pragma unroll
         for (int u = 0; u < U; ++u)
 #pragma unroll
-            for (int c = 0; c < CPL; ++c) acc[c] = madd(v[u][c], xv[u], acc[c]);
+            for (int c = 0; c < CPL; ++c) part[u % NS][c] = madd(v[u][c], xv[u], part[u % NS][c]);
+        if (SETS == 0) total();
     }
     if (j < j1) {  // the last, partial group: rows past the segment are read as its last and add nothing
         T v[U][CPL], xv[U];
@@ -118,9 +146,10 @@ __global__ void __launch_bounds__(kThreads) gemv_cols_cluster_kernel(Args a) {
         for (int u = 0; u < U; ++u) {
             const bool in = j + (size_t)u * STEP < j1;
 #pragma unroll
-            for (int c = 0; c < CPL; ++c) acc[c] = in ? madd(v[u][c], xv[u], acc[c]) : acc[c];
+            for (int c = 0; c < CPL; ++c) part[u % NS][c] = in ? madd(v[u][c], xv[u], part[u % NS][c]) : part[u % NS][c];
         }
     }
+    total();
     // rows of a warp, then warps, then segments, each in a fixed order
 #pragma unroll
     for (int off = LPR; off < 32; off <<= 1)
@@ -131,10 +160,14 @@ __global__ void __launch_bounds__(kThreads) gemv_cols_cluster_kernel(Args a) {
         for (int c = 0; c < CPL; ++c) red[w][column(c)] = acc[c];
     __syncthreads();
     if (threadIdx.x < W) {
-        T t = red[0][threadIdx.x];
+        T t[kWarps];
 #pragma unroll
-        for (int ww = 1; ww < kWarps; ++ww) t += red[ww][threadIdx.x];
-        sums[threadIdx.x] = t;
+        for (int ww = 0; ww < kWarps; ++ww) t[ww] = red[ww][threadIdx.x];
+#pragma unroll
+        for (int n = kWarps / 2; n > 0; n /= 2)
+#pragma unroll
+            for (int ww = 0; ww < n; ++ww) t[ww] = t[2 * ww] + t[2 * ww + 1];
+        sums[threadIdx.x] = t[0];
     }
     const unsigned nseg = gridDim.y;
     if (nseg > 1) tc::cluster_sync();
