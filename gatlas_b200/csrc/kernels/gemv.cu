@@ -162,6 +162,33 @@ __device__ __forceinline__ void row_strided(T (&acc)[ROWS], const V *const (&aro
     else row_last<1, STRIDE>(acc, arow, x, c, rem);
 }
 
+// Vectors c, c + STRIDE, ... of a row, U at a time and the rest one by one.
+// Written out, not through row_group: the compiler keeps more of a group's loads in
+// flight this way (doubles off the 16-byte grid, 28440 x 4085: 176 us, 219
+// through row_group), and a rest of one vector a lane costs less than row_last's
+// clamped one (30000 x 4400 floats 86 us and 91).
+template <int U, int STRIDE, typename T, typename V, int ROWS>
+__device__ __forceinline__ void row_serial(T (&acc)[ROWS], const V *const (&arow)[ROWS], const V *x, size_t c, size_t nvec) {
+    for (; c + (U - 1) * STRIDE < nvec; c += U * STRIDE) {
+        V av[ROWS][U], xv[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) xv[u] = __ldg(x + c + u * STRIDE);
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r)
+#pragma unroll
+            for (int u = 0; u < U; ++u) av[r][u] = __ldcs(arow[r] + c + u * STRIDE);
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int r = 0; r < ROWS; ++r) acc[r] = dot_acc(acc[r], av[r][u], xv[u]);
+    }
+    for (; c < nvec; c += STRIDE) {
+        const V xv = __ldg(x + c);
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) acc[r] = dot_acc(acc[r], __ldcs(arow[r] + c), xv);
+    }
+}
+
 // FEW: few warps per SM, so the tail of a row loads at once (row_tail); with
 // many its extra loads cost more (32768 x 1023: 29 us, 33 with row_tail; 1024^2
 // the other way round).
@@ -198,9 +225,7 @@ __global__ void __launch_bounds__(kGemvThreads, VW == 2 ? 5 : 0)
             static_assert(UNROLL == 4, "row_strided");
             row_strided<32>(acc, arow, x, lane, 0, nvec);
         } else {  // (row_strided: 32768 x 1023 floats 29 -> 41 us)
-            size_t c = lane;
-            for (; c + (UNROLL - 1) * 32 < nvec; c += UNROLL * 32) row_group<UNROLL, 32>(acc, arow, x, c);
-            for (; c < nvec; c += 32) row_group<1, 32>(acc, arow, x, c);
+            row_serial<UNROLL, 32>(acc, arow, x, lane, nvec);
         }
 #pragma unroll
         for (int r = 0; r < ROWS; ++r) {
@@ -229,7 +254,7 @@ __global__ void __launch_bounds__(kGemvThreads, VW == 2 ? 5 : 0)
 // fixed butterfly per warp and a fixed-order sum over the 8 warps in shared
 // memory.  The units are 8 times smaller than a warp's rows, so a 16384^2
 // product is thousands of CTAs and the last partial wave costs little.
-template <typename T, int VW, int RB, int UNROLL>
+template <typename T, int VW, int RB, int UNROLL, bool SERIAL>
 __global__ void __launch_bounds__(kGemvThreads)
     gemv_rowblock_kernel(GemvArgs a) {
     using V = typename VecT<T, VW>::type;
@@ -257,6 +282,8 @@ __global__ void __launch_bounds__(kGemvThreads)
             for (; c + (UNROLL - 1) * kGemvThreads < nvec; c += UNROLL * kGemvThreads)
                 row_group<UNROLL, kGemvThreads>(acc, arow, x, c);
             if (c < nvec) row_tail<T, V, RB, UNROLL, kGemvThreads>(acc, arow, x, c, nvec);
+        } else if constexpr (SERIAL) {
+            row_serial<UNROLL, kGemvThreads>(acc, arow, x, threadIdx.x, nvec);
         } else {
             static_assert(UNROLL == 4, "row_strided");
             row_strided<kGemvThreads>(acc, arow, x, threadIdx.x, w * 32, nvec);
@@ -649,19 +676,38 @@ static int matvec_launch(const gatlas_matvec_desc *d, const T *A, const T *x, T 
         constexpr int VWV = 16 / sizeof(T);
         const size_t per_row = vec_ok ? d->n / VWV : d->n;  // loads per row
         // long rows take a CTA per RB rows: 1024 vectors, or as many single elements
-        // unless there are rows enough for a warp each (27908 x 1287 doubles: 58 us
-        // with warps, 62 with CTAs; 3001 x 7013: 46 and 18; 7001 x 1201 floats 9 and
-        // 10, doubles 19 and 17)
-        const bool many = d->m * batch >= (size_t)sms * (sizeof(T) == 4 && per_row < (size_t)8 * kGemvThreads ? 32 : 64);
-        if (per_row >= (size_t)4 * kGemvThreads && (vec_ok || !many || per_row >= (size_t)16 * kGemvThreads)) {
+        // unless there are rows enough for a warp each.  How many that takes grows with
+        // the row (floats 7500 x 2049 10 us with warps, 14 with CTAs, 9000 x 3001 25 and
+        // 29, 9000 x 3502 31 and 30; doubles 7001 x 1201 12 and 14, 6000 x 2343 31 and 27,
+        // 9000 x 2343 36 and 39, 9000 x 3503 51 and 45; 27908 x 1287 58 and 62)
+        constexpr size_t kT = kGemvThreads;
+        const size_t rows_all = d->m * batch;
+        const size_t warps_from = (size_t)sms * (sizeof(T) == 4 ? (per_row < 8 * kT ? 32 : per_row < 13 * kT ? 27 : 64)
+                                                                : (per_row < 8 * kT ? 32 : per_row < 11 * kT ? 48 : 64));
+        // (12000 x 4501 43 and 49, 16000 x 4501 72 and 64)
+        const bool many = rows_all >= warps_from &&
+                          (per_row < 16 * kT || (sizeof(T) == 4 && per_row < 20 * kT && rows_all < (size_t)sms * 96));
+        if (per_row >= (size_t)4 * kGemvThreads && (vec_ok || !many)) {
             // (single elements: twice as many in flight where the row holds them)
             constexpr int RB = 2;
             const size_t nblocks = (d->m + RB - 1) / RB;
             const size_t cap = (size_t)sms * 64 / (batch < 8 ? batch : 8);
             dim3 g((unsigned)(nblocks < cap ? nblocks : cap), (unsigned)batch);
-            if (vec_ok) gemv_rowblock_kernel<T, VWV, RB, 4><<<g, kGemvThreads, 0, stream>>>(a);
-            else if (per_row >= (size_t)8 * kGemvThreads) gemv_rowblock_kernel<T, 1, RB, 8><<<g, kGemvThreads, 0, stream>>>(a);
-            else gemv_rowblock_kernel<T, 1, RB, 4><<<g, kGemvThreads, 0, stream>>>(a);
+            // row_serial where rows end soon after the first group (doubles: first two), by
+            // not much more than one vector a thread (15000 x 4100 floats 43.5 us, 46 through
+            // row_strided, 5264 x 5244 21 and 22; but 25164 x 8924 140 and 132, 10000 columns
+            // 81 and 76, 7200 58 and 41), doubles in few rows also after more groups (1500 x
+            // 8200 21 and 22), and long rows of them with any rest (568 x 26424 29 and 32,
+            // 1126 x 46736 72 and 71)
+            const size_t rest = per_row % (4 * kT);
+            const bool few_f64 = sizeof(T) == 8 && rows_all <= (size_t)sms * 12;
+            const bool serial = (rest > 0 && rest * 4 < 5 * kT && (per_row < (sizeof(T) == 8 ? 12 : 8) * kT || few_f64)) ||
+                                (few_f64 && rows_all <= (size_t)sms * 7 && per_row >= 32 * kT);
+            if (vec_ok && serial) gemv_rowblock_kernel<T, VWV, RB, 4, true><<<g, kGemvThreads, 0, stream>>>(a);
+            else if (vec_ok) gemv_rowblock_kernel<T, VWV, RB, 4, false><<<g, kGemvThreads, 0, stream>>>(a);
+            else if (per_row >= (size_t)8 * kGemvThreads)
+                gemv_rowblock_kernel<T, 1, RB, 8, false><<<g, kGemvThreads, 0, stream>>>(a);
+            else gemv_rowblock_kernel<T, 1, RB, 4, false><<<g, kGemvThreads, 0, stream>>>(a);
             return check_launch("gemv_rowblock_kernel");
         }
         // shorter rows: a warp per two rows, or per row (and twice the loads of
@@ -669,7 +715,7 @@ static int matvec_launch(const gatlas_matvec_desc *d, const T *A, const T *x, T 
         // of it, five CTAs per SM, and again where two rows a warp just begin a
         // second wave (N = 3500: M = 6200 13 us and 17 with two rows, 7400 22 and
         // 19, 11000 28 and 25, 13000 32 and 36, 18000 51 and 43)
-        const size_t rows_all = d->m * batch, wave = 5 * kGemvWarps * (size_t)sms;
+        const size_t wave = 5 * kGemvWarps * (size_t)sms;
         const bool few = rows_all < (size_t)sms * 4 * kGemvWarps ||
                          (vec_ok && (rows_all * 20 <= wave * (sizeof(T) == 8 ? 21 : 23) ||
                                      (rows_all > 2 * wave && rows_all * 10 <= wave * 24)));

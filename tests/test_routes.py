@@ -36,6 +36,27 @@ def _matvec_exact(cuda, engine, M, N, dtype, trans_a, kernel):
     assert torch.equal(y.double(), 2.0 * product - 3.0 * y0.double())
 
 
+# rows that end 1 vector, and just under and over 1.25 vectors a thread, after
+# whole groups of 1024; doubles in few and in many rows
+@pytest.mark.parametrize("M,N,dtype,kernel", [
+    (301, 4100, "float32", "gemv_rowblock_kernelIfLi4ELi2ELi4ELb1E"),
+    (301, 5372, "float32", "gemv_rowblock_kernelIfLi4ELi2ELi4ELb1E"),
+    (301, 5376, "float32", "gemv_rowblock_kernelIfLi4ELi2ELi4ELb0E"),
+    (33, 8196, "float32", "gemv_rowblock_kernelIfLi4ELi2ELi4ELb0E"),
+    (33, 8194, "float64", "gemv_rowblock_kernelIdLi2ELi2ELi4ELb1E"),
+    (33, 17402, "float64", "gemv_rowblock_kernelIdLi2ELi2ELi4ELb1E"),
+    (1801, 4098, "float64", "gemv_rowblock_kernelIdLi2ELi2ELi4ELb1E"),
+    (1801, 8194, "float64", "gemv_rowblock_kernelIdLi2ELi2ELi4ELb0E"),
+    (4001, 2342, "float32", "gemv_rows_kernelIfLi1E"),
+    (7105, 2343, "float64", "gemv_rows_kernelIdLi1ELi2E"),
+    (4739, 1025, "float64", "gemv_rows_kernelIdLi1ELi2E"),
+    (9473, 4501, "float32", "gemv_rows_kernelIfLi1ELi2E"),
+    (9473, 3501, "float32", "gemv_rows_kernelIfLi1ELi2E"),
+    (301, 3501, "float32", "gemv_rowblock_kernelIfLi1E")])
+def test_buffer_rows(cuda, M, N, dtype, kernel):
+    _matvec_exact(cuda, "buffer", M, N, dtype, False, kernel)
+
+
 # every column-cluster kernel, with a last block and a last segment that are not
 # whole, and one row more than a segment takes
 @pytest.mark.parametrize("M,N,dtype,kernel", [
