@@ -405,22 +405,34 @@ static bool map_fits(int64_t inner, int64_t rows, int64_t lda, size_t ts) {
 // shared memory stream as fast as loads into registers or a little faster, but
 // one CTA per SM takes whole blocks of 16 rows (or segments of a column block),
 // so its rounds have to come out even and its start has to be paid off.
-//  * rows: blocks that fill 90 % of their rounds (doubles 85), and 250 MB (25100
-//    x 3768 doubles 119 us, buffer 146; 16684 x 3720 86 and 99; 4420 x 15408
-//    floats 46 and 55; but 2788 x 28672 floats 78 and 51, 6412 x 1820 14 and 11);
+//  * rows, one round: wherever the other kernel's pairs of rows need a second
+//    wave (five CTAs per SM) and A is about as large as L2 (1700 x 30000 doubles 77
+//    us, buffer 86; 2200 x 20000 floats 31 and 33; but 1400 x 30000 76 and 57, 1900 x
+//    11184 floats, 85 MB, 18 and 14);
+//  * rows, more rounds: blocks that fill 90 % of them (doubles 85), from the same
+//    size up to three rounds, from more beyond, where rows are shorter (4716 x
+//    6360 floats 23 us and 25, 9452 x 5288 35 and 37, but 9452 x 1980 doubles, 150 MB,
+//    29 and 27, 18924 x 2640 floats 39 and 37; 25100 x 3768 doubles 119 and 146;
+//    uneven: 2788 x 28672 floats 78 and 51);
 //  * columns: doubles whose segments use 82 % of the SMs' time, from 500 MB (87 %
-//    from 380: 16164 x 6136 116 us, buffer 128; 1932 x 25208 65 and 70; but 19824 x
-//    3300 103 and 81, floats 12036 x 1448 18 and 12, 2020 x 5472 19 and 10).
+//    from 380: 18604 x 10800 226 us, buffer 233; 56388 x 3720 243 and 252; on even
+//    rounds the two differ by 2 to 8 % either way), or 70 % where no partial sums
+//    are needed (72 % from 75 MB: 15120 x 2404 47 and 49, 17452 x 580 12 and 14; but
+//    14444 x 796 17 and 14, 19824 x 3300 103 and 81, floats 12036 x 1448 18 and 12).
 template <typename T>
 static bool tiles_better(const gatlas_matvec_desc *d, int64_t M, int64_t N, int sms) {
     using namespace gvi;
     const double bytes = (double)M * (double)N * sizeof(T);
     if (!d->trans_a) {
         const int64_t blocks = (M + RB - 1) / RB, rounds = (blocks + sms - 1) / sms;
-        return bytes >= 250e6 && (double)blocks >= (sizeof(T) == 8 ? 0.85 : 0.9) * (double)(rounds * sms);
+        if (rounds == 1) return bytes >= 95e6 && (M + 1) / 2 > 5 * (int64_t)sms;
+        return bytes >= (rounds <= 3 ? 95e6 : rounds <= 6 ? 190e6 : 250e6) &&
+               (double)blocks >= (sizeof(T) == 8 ? 0.85 : 0.9) * (double)(rounds * sms);
     }
-    return sizeof(T) == 8 && bytes >= 380e6 &&
-           col_segments(M, N, sms, Elem<T>::ROW, sizeof(T)).eff >= (bytes >= 500e6 ? 0.82 : 0.87);
+    if (sizeof(T) == 4 || bytes < 75e6) return false;
+    const ColSegments s = col_segments(M, N, sms, Elem<T>::ROW, sizeof(T));
+    if (s.nseg == 1) return s.eff >= (bytes >= 250e6 ? 0.7 : 0.72);
+    return bytes >= 380e6 && s.eff >= (bytes >= 500e6 ? 0.82 : 0.87);
 }
 
 template <typename T>

@@ -36,6 +36,19 @@ def _matvec_exact(cuda, engine, M, N, dtype, trans_a, kernel):
     assert torch.equal(y.double(), 2.0 * product - 3.0 * y0.double())
 
 
+# TMA tiles: 16 rows x 256 floats or 128 doubles (rows), 32 rows x 128 doubles
+# (columns); last row block, last chunk and last segment partial
+@pytest.mark.parametrize("M,N,dtype", [(1700, 20004, "float32"), (4420, 15408, "float32"), (1601, 8002, "float64"),
+                                       (4730, 8002, "float64")])
+def test_image_rows_on_tiles(cuda, M, N, dtype):
+    _matvec_exact(cuda, "image", M, N, dtype, False, "gemv_rows_tma_kernel")
+
+
+@pytest.mark.parametrize("M,N", [(17452, 580), (2530, 21470), (130, 1001), (2, 33)])
+def test_image_columns_on_tiles(cuda, M, N):
+    _matvec_exact(cuda, "image", M, N, "float64", True, "gemv_cols_tma_kernel")
+
+
 # rows that end 1 vector, and just under and over 1.25 vectors a thread, after
 # whole groups of 1024; doubles in few and in many rows
 @pytest.mark.parametrize("M,N,dtype,kernel", [
