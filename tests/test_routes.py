@@ -9,6 +9,36 @@ from captured import kernel_names
 pytestmark = pytest.mark.gpu
 
 
+def _uniform(cuda, n, seed):
+    import torch
+    return g.fill(torch.empty(n, dtype=torch.float32, device=cuda), "uniform", seed=seed)
+
+
+# Operands off the 16-byte grid (odd K), over many 64-deep slices, so that the
+# ring and the warp groups turn; against the two-pass path bit for bit.
+@pytest.mark.parametrize("ta,tb", [(0, 0), (0, 1), (1, 1)])
+@pytest.mark.parametrize("engine,M,N,K", [("tc_bf16", 64, 50, 501), ("tc_bf16", 130, 200, 251),
+                                          ("tc_split3", 40, 70, 1501), ("tc_split3", 130, 200, 501),
+                                          ("tc_split6", 64, 100, 3001), ("tc_split6", 130, 200, 2051)])
+def test_one_launch_contraction_of_unaligned_operands(cuda, engine, ta, tb, M, N, K):
+    import torch
+    A, B = _uniform(cuda, M * K, 1), _uniform(cuda, K * N, 2)
+    one = torch.full((M * N,), float("nan"), device=cuda)
+    two = torch.full((M * N,), float("nan"), device=cuda)
+    size = g.matmul_workspace_size(M, N, K, engine, ta, tb)
+    buf = torch.empty(size + 1024, dtype=torch.uint8, device=cuda)
+    ws = buf[-buf.data_ptr() % 1024:]
+    kw = dict(trans_a=ta, trans_b=tb, engine=engine)
+    names = kernel_names(lambda: g.matmul(A, B, M, N, K, C=one, **kw))
+    assert len(names) == 1 and "tc_gemm_direct_kernel" in names[0]
+    names = kernel_names(lambda: g.matmul(A, B, M, N, K, C=two, workspace=ws, **kw))
+    assert len(names) == 2 and not any("direct" in n for n in names)
+    g.matmul(A, B, M, N, K, C=one, **kw)
+    g.matmul(A, B, M, N, K, C=two, workspace=ws, **kw)
+    assert g.device_faults() == 0
+    assert torch.equal(one, two)
+
+
 def _matvec_exact(cuda, engine, M, N, dtype, trans_a, kernel):
     """Small integers, so that every order of summation gives the same bits."""
     import torch
