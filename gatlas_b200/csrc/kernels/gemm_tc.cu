@@ -73,14 +73,19 @@ struct Params {
     // 1: A's loads evict-last in L2 (A is reused by every tile column of a
     // raster group, B by the group's tile rows at about the same time)
     int l2_hint;
-    // FP8 persistent kernel: per tile (instance-major, then tile row, then
-    // tile column) the segment count, one segment-start bit per 128-deep
-    // block (plan_words words), and each segment's scale products of the
-    // tile's two column halves (kblocks entries reserved per tile)
+    // FP8 persistent kernel: per 256 x 256 block of C (instance-major, then block
+    // row, then block column) the segment count, one segment-start bit per
+    // 128-deep block (plan_words words), and each segment's scale products of
+    // the block's two column halves, for its upper and its lower 128 rows (2 *
+    // kblocks entries reserved per block); read past L1, since the kernel may have
+    // started before they were written
     const int *plan_nseg;
     const uint32_t *plan_bits;
     const float2 *plan_q;
     int plan_words;
+    // FP8 products that either kernel may serve: 1 runs where the plan's segments
+    // are long (CTA pairs), 2 where they are short (single CTAs); 0: always
+    int when;
 };
 
 // Warp roles: warp 0 = TMA producer (lane 0), warp 1 = MMA issuer (lane 0),
@@ -96,6 +101,7 @@ constexpr int kThreadsP = 384;
 constexpr int kIssueRegs = 40, kDrainRegs = 232;
 static_assert(128 * kIssueRegs + 256 * kDrainRegs <= kThreadsP * 168, "register split");
 constexpr uint32_t kTmemCols2 = 2 * BN;  // two accumulator buffers
+constexpr int kLongRun = 8;              // blocks of K per FP8 segment from which CTA pairs are faster
 
 // Plain-store epilogue of one warp's 32 x 32 chunk (beta != 0, or rows of C off
 // the 16-byte grid, where a TMA store cannot go): v holds row `lane`'s 32
@@ -133,6 +139,21 @@ __device__ __forceinline__ void store_chunk_plain(uint8_t *stage, int lane, cons
         }
     }
     __syncwarp();  // the staging tile is read
+}
+
+// Whether an FP8 plan's segments are long: 8 blocks of K or all of it, on average
+// over an even sample of its `blocks` entries.  Every CTA of both contraction
+// kernels asks and gets the same answer.
+__device__ __forceinline__ bool plan_runs_long(const Params &p, int64_t blocks) {
+    __shared__ int warp_sum[kThreadsP / 32];
+    const int n = (int)(blocks < kThreadsP ? blocks : kThreadsP);
+    int v = (int)threadIdx.x < n ? __ldcg(p.plan_nseg + (int64_t)threadIdx.x * blocks / n) : 0;
+    v = __reduce_add_sync(0xffffffffu, v);
+    if (threadIdx.x % 32 == 0) warp_sum[threadIdx.x / 32] = v;
+    __syncthreads();
+    int total = 0;
+    for (int w = 0; w < kThreadsP / 32; ++w) total += warp_sum[w];
+    return total <= (int64_t)n * (p.kblocks > kLongRun ? p.kblocks / kLongRun : 1);
 }
 
 // ---------------------------------------------------------------------------
@@ -203,11 +224,31 @@ __global__ void __launch_bounds__(kThreadsP, 1)
         tm = first_m + r % gm;
         tn = r / gm;
     };
+    // FP8: tile -> its 256 x 256 block in the plan
+    auto plan_index = [&](int tm, int tn, int z) {
+        const int rows = PAIR ? p.tiles_m : (p.tiles_m + 1) / 2;
+        return ((int64_t)z * rows + (PAIR ? tm : tm >> 1)) * p.tiles_n + tn;
+    };
     auto wait = [&](uint64_t *bar, uint32_t parity, uint64_t limit) {  // by whole warps
         return PAIR ? tc::wait_warp_cluster(bar, parity, limit, &abort_flag)
                     : tc::wait_warp(bar, parity, limit, &abort_flag);
     };
 
+    if constexpr (MD::SCALED) {
+        if (p.when == 2) {
+            // starts while the other kernel runs, whose start the plan came before, and
+            // works, or ends, after it
+            const bool mine = !plan_runs_long(p, plan_index(0, 0, p.batch));
+            tc::wait_for_launch_before();
+            if (!mine) return;
+        } else {
+            tc::wait_for_launch_before();  // the plan
+            if (p.when == 1) {
+                tc::let_next_launch_start();
+                if (!plan_runs_long(p, plan_index(0, 0, p.batch))) return;
+            }
+        }
+    }
     if (threadIdx.x == 0) {
         for (int s = 0; s < S; ++s) {
             mbar_init(&full[s], 1);
@@ -317,16 +358,16 @@ __global__ void __launch_bounds__(kThreadsP, 1)
                 if constexpr (MD::SCALED) {
                     int tm, tn, z;
                     decode(t, tm, tn, z);
-                    wb = p.plan_bits + (((int64_t)z * p.tiles_m + tm) * p.tiles_n + tn) * p.plan_words;
-                    wcur = __ldg(wb);
-                    wnext = p.plan_words > 1 ? __ldg(wb + 1) : 0u;
+                    wb = p.plan_bits + plan_index(tm, tn, z) * p.plan_words;
+                    wcur = __ldcg(wb);
+                    wnext = p.plan_words > 1 ? __ldcg(wb + 1) : 0u;
                 }
                 for (int kb = 0; kb < p.kblocks; ++kb) {
                     bool seg_first, seg_last;
                     if constexpr (MD::SCALED) {
                         if (kb > 0 && (kb & 31) == 0) {  // next word; the one after it loads meanwhile
                             wcur = wnext;
-                            wnext = (kb >> 5) + 1 < p.plan_words ? __ldg(wb + (kb >> 5) + 1) : 0u;
+                            wnext = (kb >> 5) + 1 < p.plan_words ? __ldcg(wb + (kb >> 5) + 1) : 0u;
                         }
                         const int k1 = kb + 1;
                         seg_first = ((wcur >> (kb & 31)) & 1u) != 0;
@@ -413,21 +454,25 @@ __global__ void __launch_bounds__(kThreadsP, 1)
             int tile_nseg = nseg;
             const float2 *tile_q = nullptr;
             if constexpr (MD::SCALED) {
-                const int64_t pidx = ((int64_t)z * p.tiles_m + tm) * p.tiles_n + tn;
-                tile_nseg = __ldg(p.plan_nseg + pidx);
-                // a pair's plan holds the products of both CTAs' rows per segment
-                tile_q = p.plan_q + pidx * p.kblocks * (PAIR ? 2 : 1) + (PAIR ? rank : 0);
+                const int64_t pidx = plan_index(tm, tn, z);
+                tile_nseg = __ldcg(p.plan_nseg + pidx);
+                // the plan holds the products of both 128-row halves per segment
+                tile_q = p.plan_q + pidx * p.kblocks * 2 + (PAIR ? (int)rank : tm & 1);
             }
             float acc[BN / 2];
 #pragma unroll
             for (int j = 0; j < BN / 2; ++j) acc[j] = 0.0f;
+            float2 q = make_float2(0.0f, 0.0f);
+            if constexpr (MD::SCALED)
+                if (tile_nseg > 0) q = __ldcg(tile_q);
             for (int g = 0; g < tile_nseg; ++g) {
                 ++seg;
                 const int b = seg & 1;
                 float scale = 1.0f;
                 if constexpr (MD::SCALED) {
-                    const float2 q = __ldg(tile_q + (PAIR ? 2 * g : g));  // this half's scale block product
+                    // this half's scale block product, read a segment ahead
                     scale = half ? q.y : q.x;
+                    if (g + 1 < tile_nseg) q = __ldcg(tile_q + 2 * g + 2);
                 }
                 if (!wait(&tfull[b], (uint32_t)(seg >> 1) & 1u, 2 * kWaitNs)) {
                     if (!abort_flag) report_fault(p.fault, kFaultTcEpilogueWait);
@@ -939,6 +984,7 @@ __global__ void __launch_bounds__(kQThreads, 3) quant_fp8_kernel(const __grid_co
     __shared__ uint32_t qt[kQBlock * 32];
     __shared__ float red[kQThreads / 32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    tc::let_next_launch_start();
     const bool second = blockIdx.x >= args.split;
     const QuantOperand &a = args.op[second ? 1 : 0];
     const int64_t block = (int64_t)blockIdx.x - (second ? args.split : 0);
@@ -1188,9 +1234,9 @@ static WsPtrs ws_ptrs(const Plan &pl, void *ws) {
 // Tiling of C for M > 128 ("tc_pair"): 1 = what measures fastest on B200 --
 // CTA pairs for the split engines (17-19 % fewer cycles per 8192^3 launch
 // than 128 x 256 single CTAs), 256 x 256 single-CTA tiles for one-product
-// BF16 over all of K (35 % fewer); FP8 on CTA pairs once every pair of SMs has
-// a tile (8192^3 398 us against 454 on single CTAs, 4096^3 84 and 90, but
-// 2048^3 26.1 and 25.2); 2 = CTA pairs always; 0 = 128 x 256 always.
+// BF16 over all of K (35 % fewer); FP8 on CTA pairs or single CTAs by the
+// length of its segments (see launch_tc); 2 = CTA pairs always; 0 = 128 x 256
+// always.
 static int g_tc_pair = 1;
 // Rows of C per raster group of the persistent kernels (multiple of 128).
 static int g_tc_group_rows = kGroupM * 128;
@@ -1199,24 +1245,23 @@ static int g_tc_group_rows = kGroupM * 128;
 // same speed.
 static int g_tc_l2_hint = 1;
 
-// FP8 segment plan, one warp per tile, 32 blocks of K at a time: a run of at
-// most seg_kblocks 128-deep blocks whose scale products sa * sb are equal for
-// every 128 x 128 block of the 256 x 256 block the tile lies in accumulates in
-// TMEM and is promoted, scaled once (exact: the scales are powers of two).
-// Writes the tile's segment count, its segment-start bits and each segment's
-// scale products.  Single CTAs (pair == 0) have 128 x 256 tiles: one A block,
-// two column halves, products (a b0, a b1) per segment.  CTA pairs (pair == 1)
-// have 256 x 256 tiles, whose MMAs share their segments: per segment the plan
-// holds (a0 b0, a0 b1) for the leader's rows and (a1 b0, a1 b1) for the
-// peer's.  Runs end where any of the four products changes in either case, so
-// both tilings promote alike and give identical results.  (One thread per tile
-// walking K serially took 6.6 us of a 4096^3 product.)
+// FP8 segment plan, one warp per 256 x 256 block of C, 32 blocks of K at a time:
+// a run of at most seg_kblocks 128-deep blocks whose scale products sa * sb are
+// equal for all four 128 x 128 quarters accumulates in TMEM and is promoted,
+// scaled once (exact: the scales are powers of two).  Writes the block's segment
+// count, its segment-start bits and each segment's scale products: (a0 b0, a0 b1)
+// for the upper rows, (a1 b0, a1 b1) for the lower.  A CTA pair's tile is such a
+// block, a single CTA's its upper or lower half, so both tilings promote alike
+// and give identical results.  (One thread per tile walking K serially took 6.6 us
+// of a 4096^3 product.)
 constexpr int kPlanWarps = 4;
 
 __global__ void __launch_bounds__(32 * kPlanWarps)
     fp8_plan_kernel(const float *scale_a, const float *scale_b, int64_t sa_stride, int64_t sb_stride, int tiles_m,
                     int tiles_n, int batch, int kblocks, int nblocks_m, int nblocks_n, int seg_kblocks, int words,
-                    int pair, int *nseg, uint32_t *bits, float2 *q) {
+                    int *nseg, uint32_t *bits, float2 *q) {
+    tc::wait_for_launch_before();  // the scales, and the last reader of this plan's memory
+    tc::let_next_launch_start();
     const int lane = threadIdx.x & 31;
     const int64_t idx = (int64_t)blockIdx.x * kPlanWarps + (threadIdx.x >> 5);
     if (idx >= (int64_t)tiles_m * tiles_n * batch) return;
@@ -1224,14 +1269,14 @@ __global__ void __launch_bounds__(32 * kPlanWarps)
     const int64_t rest = idx / tiles_n;
     const int tm = (int)(rest % tiles_m);
     const int64_t z = rest / tiles_m;
-    const int ma0 = pair ? 2 * tm : tm & ~1, ma1 = ma0 + 1;
+    const int ma0 = 2 * tm, ma1 = ma0 + 1;
     const float *sa0 = scale_a + z * sa_stride + (int64_t)ma0 * kblocks;
     const float *sa1 = ma1 < nblocks_m ? scale_a + z * sa_stride + (int64_t)ma1 * kblocks : nullptr;
     const int nb0 = 2 * tn, nb1 = 2 * tn + 1;
     const float *sb0 = nb0 < nblocks_n ? scale_b + z * sb_stride + (int64_t)nb0 * kblocks : nullptr;
     const float *sb1 = nb1 < nblocks_n ? scale_b + z * sb_stride + (int64_t)nb1 * kblocks : nullptr;
     uint32_t *wb = bits + idx * words;
-    float2 *qt = q + idx * kblocks * (pair ? 2 : 1);
+    float2 *qt = q + idx * kblocks * 2;
     int count = 0, run0 = 0;                       // segments so far; first block of the run of equal products
     float carry[4] = {0.0f, 0.0f, 0.0f, 0.0f};     // the products of the block before this word
     for (int w = 0; w < words; ++w) {
@@ -1255,12 +1300,8 @@ __global__ void __launch_bounds__(32 * kPlanWarps)
         const uint32_t starts = __ballot_sync(0xffffffffu, start);
         if (start) {
             const int s = count + __popc(starts & ((1u << lane) - 1u));
-            if (pair) {
-                qt[2 * s] = make_float2(cur[0], cur[1]);
-                qt[2 * s + 1] = make_float2(cur[2], cur[3]);
-            } else {
-                qt[s] = tm & 1 ? make_float2(cur[2], cur[3]) : make_float2(cur[0], cur[1]);
-            }
+            qt[2 * s] = make_float2(cur[0], cur[1]);
+            qt[2 * s + 1] = make_float2(cur[2], cur[3]);
         }
         if (lane == 0) wb[w] = starts;
         count += __popc(starts);
@@ -1287,6 +1328,15 @@ static void c_tensor_map(const Geometry &g, Params &p, CUtensorMap *tcout) {
 // Persistent launch: as many CTAs (CTA pairs) as fit on the GPU at once, at
 // most one per tile.  C leaves through a TMA tensor map unless beta is used
 // or C is not 16-byte aligned in rows and instances.
+// A launch that may start while the one before it still runs, as far as that
+// one lets it; the kernel waits for it (tc::wait_for_launch_before).
+static cudaLaunchAttribute early_start() {
+    cudaLaunchAttribute a;
+    a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    a.val.programmaticStreamSerializationAllowed = 1;
+    return a;
+}
+
 template <int MODE, bool PAIR>
 static int launch_persistent(const CUtensorMap *ta, const CUtensorMap *tb, const Geometry &g, Params p,
                              cudaStream_t stream) {
@@ -1310,13 +1360,16 @@ static int launch_persistent(const CUtensorMap *ta, const CUtensorMap *tb, const
     cfg.blockDim = dim3(kThreadsP, 1, 1);
     cfg.dynamicSmemBytes = (size_t)smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = PAIR ? 2 : 1;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
+    cudaLaunchAttribute attr[2];
     cfg.attrs = attr;
-    cfg.numAttrs = PAIR ? 1 : 0;
+    if (PAIR) {
+        cudaLaunchAttribute &a = attr[cfg.numAttrs++];
+        a.id = cudaLaunchAttributeClusterDimension;
+        a.val.clusterDim.x = 2;
+        a.val.clusterDim.y = 1;
+        a.val.clusterDim.z = 1;
+    }
+    if (MODE == 3) attr[cfg.numAttrs++] = early_start();
     // resident units: CTAs (one per SM) or clusters of two, as the occupancy query reports
     static thread_local int cap_dev = -1, cap = 0;
     int dev = 0;
@@ -1374,26 +1427,33 @@ template <int MODE>
 static int launch_tc(const Geometry &g, const Plan &pl, const WsPtrs &w, float *C, double alpha, double beta,
                      int gemm, uint32_t extra, cudaStream_t stream) {
     using L = Layout<MODE>;
-    const int64_t pair_tiles = ((g.M + 2 * BM - 1) / (2 * BM)) * ((g.N + BN - 1) / BN) * g.batch;
-    const bool pair = g.M > BM && (g_tc_pair == 2 || (g_tc_pair == 1 && (MODE == 1 || MODE == 2 ||
-                                                                         (MODE == 3 && pair_tiles >= sm_count() / 2))));
+    const bool pair = g.M > BM && (g_tc_pair == 2 || (g_tc_pair == 1 && (MODE == 1 || MODE == 2)));
     CUtensorMap ta[3], tb[3];
     const uint64_t row_bytes = (uint64_t)pl.Kp * pl.elem;
     const uint64_t adims[3] = {(uint64_t)pl.Kp, (uint64_t)g.M, (uint64_t)g.batch};
     const uint64_t astr[2] = {row_bytes, row_bytes * (uint64_t)g.M};
     const uint64_t bdims[3] = {(uint64_t)pl.Kp, (uint64_t)g.N, (uint64_t)g.batch};
     const uint64_t bstr[2] = {row_bytes, row_bytes * (uint64_t)g.N};
-    // a CTA of a pair stages 128 rows of B (its half of the pair's 256 columns)
-    const uint32_t abox[3] = {(uint32_t)L::BK, BM, 1}, bbox[3] = {(uint32_t)L::BK, pair ? 128u : (uint32_t)BN, 1};
+    const uint32_t abox[3] = {(uint32_t)L::BK, BM, 1};
     const CUtensorMapDataType dt = MODE == 3 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
     const CUtensorMapSwizzle swz = L::ROW_BYTES == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B;
     for (int i = 0; i < 3; ++i) {
         const int src = i < pl.np ? i : 0;  // unused slots alias piece 0
         int rc = make_tensor_map(&ta[i], dt, 3, w.a[src], adims, astr, abox, swz);
         if (rc) return rc;
-        rc = make_tensor_map(&tb[i], dt, 3, w.b[src], bdims, bstr, bbox, swz);
         if (rc) return rc;
     }
+    // a CTA of a pair stages 128 rows of B (its half of the pair's 256 columns)
+    auto b_maps = [&](bool half) {
+        const uint32_t box[3] = {(uint32_t)L::BK, half ? 128u : (uint32_t)BN, 1};
+        for (int i = 0; i < 3; ++i) {
+            const int rc = make_tensor_map(&tb[i], dt, 3, w.b[i < pl.np ? i : 0], bdims, bstr, box, swz);
+            if (rc) return rc;
+        }
+        return (int)GATLAS_OK;
+    };
+    int rc = b_maps(pair);
+    if (rc) return rc;
     Params p;
     std::memset(&p, 0, sizeof(p));
     p.C = C;
@@ -1426,23 +1486,45 @@ static int launch_tc(const Geometry &g, const Plan &pl, const WsPtrs &w, float *
         return pair ? launch_persistent<MODE, true>(ta, tb, g, p, stream)
                     : launch_persistent<MODE, false>(ta, tb, g, p, stream);
     } else {
-        // plan every tile's segments (256 x 256 tiles on CTA pairs, 128 x 256
-        // on single CTAs), then the persistent kernel
-        const int64_t tm_rows = pair ? 2 * BM : BM;
-        const int64_t tiles_m = (g.M + tm_rows - 1) / tm_rows, tiles_n = (g.N + BN - 1) / BN;
+        // plan the segments of every 256 x 256 block, then the persistent kernel
+        const int64_t tiles_m = (g.M + 2 * BM - 1) / (2 * BM), tiles_n = (g.N + BN - 1) / BN;
         const int64_t tiles = tiles_m * tiles_n * g.batch;
         if (tiles > 0) {
             const int words = (int)((p.kblocks + 31) / 32);
-            fp8_plan_kernel<<<(unsigned)((tiles + kPlanWarps - 1) / kPlanWarps), 32 * kPlanWarps, 0, stream>>>(
-                w.sa, w.sb, p.scale_a_stride, p.scale_b_stride, (int)tiles_m, (int)tiles_n, (int)g.batch,
-                p.kblocks, p.nblocks_m, p.nblocks_n, p.seg_kblocks, words, pair ? 1 : 0, w.plan_nseg, w.plan_bits,
-                w.plan_q);
-            int rc = check_launch("fp8_plan_kernel");
-            if (rc) return rc;
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3((unsigned)((tiles + kPlanWarps - 1) / kPlanWarps), 1, 1);
+            cfg.blockDim = dim3(32 * kPlanWarps, 1, 1);
+            cfg.stream = stream;
+            cudaLaunchAttribute attr = early_start();
+            cfg.attrs = &attr;
+            cfg.numAttrs = 1;
+            const cudaError_t e = cudaLaunchKernelEx(
+                &cfg, fp8_plan_kernel, (const float *)w.sa, (const float *)w.sb, p.scale_a_stride, p.scale_b_stride,
+                (int)tiles_m, (int)tiles_n, (int)g.batch, p.kblocks, p.nblocks_m, p.nblocks_n, p.seg_kblocks, words,
+                w.plan_nseg, w.plan_bits, w.plan_q);
+            if (e != cudaSuccess) return set_error(GATLAS_ERR_CUDA, "fp8_plan_kernel: %s", cudaGetErrorString(e));
             p.plan_nseg = w.plan_nseg;
             p.plan_bits = w.plan_bits;
             p.plan_q = w.plan_q;
             p.plan_words = words;
+        }
+        // With two tiles for every pair of SMs, pairs are faster where segments are
+        // long (contraction of 4096^3 uniform operands 60 us, single CTAs 66; 8192 x 8192
+        // x 1024 85 and 92, but x 512 73 and 64) and much slower where they are short,
+        // since a promotion is a round trip between the two CTAs (scales that change
+        // with every block, 4096^3 161 us and 91, 8192^3 1060 and 550; every fourth 75
+        // both).  Only the device knows the scales, so both kernels are launched and
+        // one of them leaves; that takes 2 us, which the launches of this engine make up
+        // by starting early (2048^3 33 -> 29 us in all).
+        const bool either = g_tc_pair == 1 && tiles >= sm_count() && p.kblocks >= kLongRun;
+        if (either) {
+            p.when = 1;
+            rc = b_maps(true);
+            if (!rc) rc = launch_persistent<MODE, true>(ta, tb, g, p, stream);
+            if (!rc) rc = b_maps(false);
+            if (rc) return rc;
+            p.when = 2;
+            return launch_persistent<MODE, false>(ta, tb, g, p, stream);
         }
         return pair ? launch_persistent<MODE, true>(ta, tb, g, p, stream)
                     : launch_persistent<MODE, false>(ta, tb, g, p, stream);
@@ -1542,11 +1624,11 @@ static int run_rows(const gatlas_matmul_desc *d, const Plan &pl, const Geometry 
     for (int i = 0; i < 3; ++i)
         if (wb.a[i]) wb.a[i] = static_cast<uint8_t *>(wb.a[i]) + r0 * pl.Kp * pl.elem;
     if (wb.sa) wb.sa += (r0 / kQBlock) * pl.kblocks;
-    if (pl.mode == 3) {  // the block's tiles in the plan of the whole product
-        const int64_t first = (r0 / BM) * ((g.N + BN - 1) / BN);
+    if (pl.mode == 3) {  // the rows' 256 x 256 blocks in the plan of the whole product
+        const int64_t first = (r0 / (2 * BM)) * ((g.N + BN - 1) / BN);
         wb.plan_nseg += first;
         wb.plan_bits += first * ((pl.kblocks + 31) / 32);
-        wb.plan_q += first * pl.kblocks;
+        wb.plan_q += first * pl.kblocks * 2;
     }
     float *Cb = C + r0 * g.ldc;
     switch (pl.mode) {

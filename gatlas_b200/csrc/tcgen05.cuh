@@ -208,19 +208,23 @@ __device__ __forceinline__ void cluster_sync() {
 
 // mbarrier wait with cluster-scope acquire (the barrier receives arrivals
 // from the other CTA of the pair), bounded in wall time.
+__device__ __forceinline__ bool try_wait_cluster(uint64_t *bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
 __device__ __forceinline__ bool wait_timed_cluster(uint64_t *bar, uint32_t parity, uint64_t limit_ns,
                                                    volatile int *abort) {
+    if (try_wait_cluster(bar, parity)) return true;
     const uint64_t t0 = globaltimer();
     while (true) {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(smem_u32(bar)), "r"(parity)
-            : "memory");
-        if (ok) return true;
+        if (try_wait_cluster(bar, parity)) return true;
         if (abort && *abort) return false;
         if (globaltimer() - t0 > limit_ns) return false;
     }
@@ -230,6 +234,12 @@ __device__ __forceinline__ bool wait_warp_cluster(uint64_t *bar, uint32_t parity
                                                   volatile int *abort) {
     return __all_sync(0xffffffffu, wait_timed_cluster(bar, parity, limit_ns, abort));
 }
+
+// Launches on one stream that overlap (programmatic dependent launch): the next
+// one may start once every CTA of this one has said so or ended; it waits until
+// this one has ended and its writes are visible.
+__device__ __forceinline__ void let_next_launch_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_launch_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Arrive on an mbarrier of another CTA of the cluster (shared::cluster address).
 __device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {

@@ -205,8 +205,9 @@ int gatlas_matmul_f32_host(const gatlas_matmul_desc *d, const float *A, const fl
  * tile C.  1 (default): CTA pairs (cta_group::2, a 256 x 256 tile per pair,
  * each CTA staging half of B) for split3 and split6; 256 x 256 tiles on
  * single CTAs for one-product BF16 over all of K once there are at least as
- * many such tiles as SMs; CTA pairs for FP8 once there are as many 256 x 256
- * tiles as SM pairs; one CTA per 128 x 256 tile otherwise.  2: CTA
+ * many such tiles as SMs; CTA pairs for FP8 from as many 256 x 256 tiles as
+ * SMs where runs of equally scaled blocks are 8 or longer on average, which the
+ * device decides; one CTA per 128 x 256 tile otherwise.  2: CTA
  * pairs always.  0: 128 x 256 tiles always.  Results are bit-identical in
  * every case (same pieces, same MMA order, same promotion).
  * "tc_group_rows": rows of C per raster group of the persistent
