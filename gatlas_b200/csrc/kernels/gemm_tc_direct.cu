@@ -542,12 +542,13 @@ Source source(const float *p, int64_t ld, int64_t rows, int64_t stride, int64_t 
 // and of width 64 take 0.40 / 0.62 / 0.87 (BF16), 0.52 / 0.72 / 1.07 (split3)
 // and 0.75 / 1.05 / 1.42 (split6), about twice that where an operand has to be
 // read in pairs, and 5 per further wave of tiles; the two-pass contraction
-// 0.30 / 0.85 / 1.85 on its wider tiles, after a split pass at 4 TB/s and two
-// more launches.  Either side of the line, direct against two-pass: 64 x 4096
-// x 8192 BF16 56 and 86 us, split3 69 and 200, split6 100 and 351; 1024^3
-// split3 21 and 27, BF16 18 and 16; 512^3 BF16 9.5 and 12.8; 1000 x 777 x 1100
-// BF16 18 and 22; 1536^3 split3 54 and 37; 128 x 128 x 4096 BF16 39 and 28;
-// 64 x 4095 x 8191 BF16 (pairs) 127 and 103; 2000 x 2000 x 100 BF16 24 and 13.
+// 0.30 / 0.85 / 1.85 on its wider tiles, after a split pass at 6.3 TB/s (5.0 where
+// an operand is stored across k) and two more launches.  Either side of the
+// line, direct against two-pass: 64 x 4096 x 8192 BF16 56 and 86 us, split3 69 and
+// 200, split6 100 and 351; 1024^3 split3 21 and 27, BF16 18 and 16; 512^3 BF16 9.5
+// and 12.8; 1000 x 777 x 1100 BF16 18 and 22; 1536^3 split3 54 and 37; 128 x 128 x
+// 4096 BF16 39 and 28; 64 x 4095 x 8191 BF16 (pairs) 127 and 103; 2000 x 2000 x 100
+// BF16 24 and 13; seven of 16 x 3688 x 3320 BF16 183 and 133.
 int direct_width(const gatlas_matmul_desc *d, const Geometry &g, const float *A, const float *B, const float *C) {
     using namespace direct;
     if (d->engine == GATLAS_ENGINE_TC_FP8) return 0;  // block scales need whole 128 x 128 blocks first
@@ -568,10 +569,11 @@ int direct_width(const gatlas_matmul_desc *d, const Geometry &g, const float *A,
         return 4.0 + w * slices * per_slice + (w - 1) * 5.0;
     };
     const bool pair = mode != 0 && g.M > BM;
-    const double elems = (double)g.batch * (double)g.K * (double)(g.M + g.N);
+    const double k_bytes = (double)g.batch * (double)g.K * (4 + 2 * (mode + 1));
+    const double split_us = k_bytes * ((double)g.M / (g.ta ? 5.0e6 : 6.3e6) + (double)g.N / (g.tb ? 6.3e6 : 5.0e6));
     // C by plain stores (beta, or rows not 16-byte aligned): 1 us per MB
     const bool plain_c = (d->gemm && d->beta != 0.0) || g.ldc % 4 != 0 || !aligned16(C) || (g.batch > 1 && g.stride_c % 4 != 0);
-    const double two_pass_us = 9.0 + elems * (4 + 2 * (mode + 1)) / 4e6 +
+    const double two_pass_us = 9.0 + split_us +
                                waves(tiles(pair ? 256 : 128, 256), pair ? sms / 2 : sms) * slices * kTwoPass[mode] +
                                (plain_c ? (double)g.batch * (double)g.M * (double)g.N * 4 * 1e-6 : 0.0);
     const double us32 = direct_us(32), us64 = g.M <= 64 ? us32 : direct_us(64);

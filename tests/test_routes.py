@@ -39,6 +39,17 @@ def test_one_launch_contraction_of_unaligned_operands(cuda, engine, ta, tb, M, N
     assert torch.equal(one, two)
 
 
+# Several waves of tiles re-reading large operands: the split pass is cheaper.
+@pytest.mark.parametrize("engine,M,N,K,batch,ta,tb", [("tc_bf16", 16, 3688, 3320, 7, 1, 1),
+                                                      ("tc_split3", 2580, 152, 2588, 8, 1, 0)])
+def test_large_operands_are_split_first(cuda, engine, M, N, K, batch, ta, tb):
+    import torch
+    A, B = _uniform(cuda, batch * M * K, 1), _uniform(cuda, batch * K * N, 2)
+    C = torch.empty(batch * M * N, device=cuda)
+    names = kernel_names(lambda: g.matmul(A, B, M, N, K, C=C, trans_a=ta, trans_b=tb, engine=engine, batch=batch))
+    assert len(names) == 2 and "split_kernel" in names[0]
+
+
 def _matvec_exact(cuda, engine, M, N, dtype, trans_a, kernel):
     """Small integers, so that every order of summation gives the same bits."""
     import torch
