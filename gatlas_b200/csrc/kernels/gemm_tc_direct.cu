@@ -555,6 +555,8 @@ int direct_width(const gatlas_matmul_desc *d, const Geometry &g, const float *A,
     // split6 counts promotion intervals in slices of 32, two to a slice here
     if (d->engine == GATLAS_ENGINE_TC_SPLIT6 && d->extra % 2 != 0) return 0;
     if (g.M > (1 << 20) || g.N > (1 << 20) || g.K > (1 << 24)) return 0;
+    // K beyond the transposing split's grid stays refused there
+    if ((g.ta || !g.tb) && g.K > 65535 * 64) return 0;
     const int mode = d->engine == GATLAS_ENGINE_TC_BF16 ? 0 : d->engine == GATLAS_ENGINE_TC_SPLIT3 ? 1 : 2;
     static const double kDirect[3][3] = {{0.40, 0.62, 0.87}, {0.52, 0.72, 1.07}, {0.75, 1.05, 1.42}};
     static const double kPairs[3] = {2.2, 1.9, 1.45}, kTwoPass[3] = {0.30, 0.85, 1.85};

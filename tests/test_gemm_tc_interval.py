@@ -40,3 +40,21 @@ def test_intervals_at_the_ends_of_the_range(cuda, engine, M, N, workspace):
     for extra in (LARGEST - 1, LARGEST):
         assert np.array_equal(_product(cuda, engine, M, N, K, extra, workspace), whole)
     assert np.array_equal(whole, _product(cuda, engine, M, N, K, 64, not workspace))
+
+
+@pytest.mark.parametrize("ta,tb", [(1, 1), (0, 0), (0, 1)])
+def test_depth_beyond_the_transposing_split_is_refused_either_way(cuda, ta, tb):
+    """An operand stored across k is split in a grid of 65535 tiles of 64 k; with
+    and without a workspace the answer is the same (both along k: accepted)."""
+    import torch
+    K = 65535 * 64 + 8
+    A, B = torch.ones(K, device=cuda), torch.ones(K, device=cuda)
+    size = g.matmul_workspace_size(1, 1, K, "tc_split3", ta, tb)
+    buf = torch.empty(size + 1024, dtype=torch.uint8, device=cuda)
+    for ws in (None, buf[-buf.data_ptr() % 1024:]):
+        if ta or not tb:
+            with pytest.raises(g.GatlasError, match="too large"):
+                g.matmul(A, B, 1, 1, K, trans_a=ta, trans_b=tb, engine="tc_split3", workspace=ws)
+        else:
+            C = g.matmul(A, B, 1, 1, K, trans_a=ta, trans_b=tb, engine="tc_split3", workspace=ws)
+            assert abs(float(C) - K) <= 2.0 ** -24 * K * (K // 256) ** 0.5
