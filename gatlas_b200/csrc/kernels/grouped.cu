@@ -842,10 +842,20 @@ int grouped_build(int engine, const gatlas_grouped_instance *in, int32_t count, 
     t->pair = g_pair_mode.load() == 1;
     // the widest access to C that every instance takes
     uint64_t low = 0;  // bits set in any N, ldc or C (in floats)
+    int64_t c_elems = 0;
+    bool reads_c = false;
     for (int i = 0; i < count; ++i)
-        if (in[i].m > 0 && in[i].n > 0)
+        if (in[i].m > 0 && in[i].n > 0) {
             low |= (uint64_t)t->ip[i].N | (uint64_t)t->ip[i].ldc | reinterpret_cast<uintptr_t>(in[i].c) >> 2;
+            c_elems += (int64_t)in[i].m * in[i].n;
+            reads_c = reads_c || (in[i].gemm && in[i].beta != 0.0);
+        }
     t->vec = low & 1 ? 1 : low & 2 ? 2 : 4;
+    // Written only, and more than L2 holds: one float a lane, a whole row of a chunk
+    // per access.  Two rows per access leave more sectors of rows off the 16-byte
+    // grid for later (148 products of 1024 x 1022 x 128 BF16 208 us, 243 with pairs;
+    // 256 of 256 x 254 x 256, in L2, 39 and 34).
+    if (t->vec == 2 && !reads_c && c_elems > (32ll << 20)) t->vec = 1;
     const int step_m = t->pair ? 2 : 1;
     size_t off = 0;
     for (int i = 0; i < count; ++i) {
