@@ -337,11 +337,12 @@ std::ostream &KernelMatmul::print(std::ostream &os) const {
        << " GEMM=" << generalizedMatmul() << " packed=" << packedCalc() << "\n";
     if (variant_ == Variant::TcFp8) {
         os << "// quant_fp8_kernel: E4M3 codes with one power-of-two FP32 scale per 128x128 block\n"
-           << "// fp8_plan_kernel: per 128x256 tile, runs of up to " << (extraParam() ? extraParam() : 4)
+           << "// fp8_plan_kernel: per 256x256 block, runs of up to " << (extraParam() ? extraParam() : 16)
            << " equally scaled 128-deep blocks\n"
-           << "// tcgen05 kernel tc_gemm_persistent_kernel<tcfp8>: one CTA per SM over 128x256 output tiles, TMA "
-           << "128B-swizzled E4M3 tiles (BK=128), tcgen05.mma kind::f8f6f4 M=128 N=256 K=32, each run promoted "
-           << "scaled into FP32 registers, C stored through TMA\n";
+           << "// tcgen05 kernel tc_gemm_persistent_kernel<tcfp8>: one CTA per SM over 128x256 output tiles (CTA pairs "
+           << "over 256x256 tiles for large products whose runs are long), TMA 128B-swizzled E4M3 tiles (BK=128), "
+           << "tcgen05.mma kind::f8f6f4 N=256 K=32, each run promoted scaled into FP32 registers, C stored through "
+           << "TMA\n";
     } else if (is_tc(variant_)) {
         const bool split6 = variant_ == Variant::TcSplit6, bf16 = variant_ == Variant::TcBf16;
         os << "// tcgen05 kernel tc_gemm_persistent_kernel<" << variant_name(variant_)

@@ -67,10 +67,10 @@ int matmul_dmma(const gatlas_matmul_desc *d, const Geometry &g, const double *A,
     a.tiles_m = a.tiles_n = 0;
     auto tiles = [&](int bm, int bn) { return ((g.M + bm - 1) / bm) * ((g.N + bn - 1) / bn) * g.batch; };
     const double c64 = tiling_cost(tiles(64, 64), 64 * 64, 33.4);
-    const double c48 = tiling_cost(tiles(64, 32), 64 * 32, 30.9);
+    const double c64x32 = tiling_cost(tiles(64, 32), 64 * 32, 30.9);
     const double c32 = tiling_cost(tiles(32, 32), 32 * 32, 29.3);
-    if (c64 <= c48 && c64 <= c32) return launch_layout<64, 64, 32, 32>(g, a, stream);
-    if (c48 <= c32) return launch_layout<64, 32, 32, 16>(g, a, stream);
+    if (c64 <= c64x32 && c64 <= c32) return launch_layout<64, 64, 32, 32>(g, a, stream);
+    if (c64x32 <= c32) return launch_layout<64, 32, 32, 16>(g, a, stream);
     return launch_layout<32, 32, 16, 16>(g, a, stream);
 }
 

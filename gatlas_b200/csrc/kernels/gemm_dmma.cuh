@@ -148,7 +148,6 @@ __global__ void __launch_bounds__(BM / WM *(BN / WN) * 32, BM *BN >= 64 * 32 ? 3
         asm volatile("cp.async.commit_group;" ::: "memory");
     }
 
-
     double acc[MI][NI][4];
 #pragma unroll
     for (int i = 0; i < MI; ++i)

@@ -13,10 +13,10 @@
 //     operands whose stored layout is not K-major;
 //  2. contraction (BF16, split3, split6): a persistent kernel, one CTA per
 //     SM over 128 x 256 tiles of C, or one cluster of two CTAs per SM pair
-//     over 256 x 256 tiles (cta_group::2).  Warp 0 lane 0 streams K slices
+//     over 256 x 256 tiles (cta_group::2).  Warp 0 streams K slices
 //     of 128 bytes per row (64 BF16; 64 bytes for split6) of every piece
 //     of A and B with 3-D TMA tensor-map loads (128-byte swizzle) into a
-//     multi-stage mbarrier ring; warp 1 lane 0 issues tcgen05.mma kind::f16
+//     multi-stage mbarrier ring; warp 1 issues tcgen05.mma kind::f16
 //     (M = 128 or 256, N = 256, K = 16) for each product of pieces (hi*hi,
 //     hi*lo, lo*hi for 3 products; the six leading products of three pieces
 //     for 6), accumulating in FP32 in two TMEM buffers of 256 columns; eight
@@ -24,7 +24,7 @@
 //     and, at the end of a tile, apply C = fma(alpha, acc, beta*C) and store
 //     C through TMA while the next tile already runs.  FP8 E4M3 (per-block
 //     scales) runs the same persistent kernel, on single CTAs or pairs, its
-//     segments planned per tile by fp8_plan_kernel.
+//     segments planned per 256 x 256 block of C by fp8_plan_kernel.
 // Every mbarrier wait is bounded in wall time; a timeout sets the device
 // fault word, stops the pipeline, drains the copies in flight and frees TMEM.
 #include <cuda.h>
@@ -88,9 +88,10 @@ struct Params {
     int when;
 };
 
-// Warp roles: warp 0 = TMA producer (lane 0), warp 1 = MMA issuer (lane 0),
-// warps 2..9 = accumulator drain + epilogue.  Drain warp w reads TMEM lane
-// quarter (w % 4) and column half (w - 2) / 4.
+// Warp roles of the wide kernel: warp 0 = TMA producer, warp 1 = MMA issuer (all
+// lanes walk and wait, an elected lane issues), warps 2..9 = accumulator drain +
+// epilogue.  Drain warp w reads TMEM lane quarter (w % 4) and column half (w - 2)
+// / 4.
 constexpr int kDrainWarps = 8;
 constexpr int kThreads2 = 32 * (2 + kDrainWarps);
 // The persistent kernel's roles are whole warpgroups: warps 0 and 1 as above (2

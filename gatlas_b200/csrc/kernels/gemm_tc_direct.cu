@@ -111,8 +111,8 @@ struct Cfg {
     static_assert(128 * PITCH * 4 <= (int)(STAGES * STAGE), "C staging fits the ring");
 };
 
-// Splits 8 values into NP words of 4 packed BF16 pairs each (the pieces of
-// split_value, two at a time).
+// Splits two values into NP words of a BF16 pair each (the pieces of
+// split_value).
 template <int NP>
 __device__ __forceinline__ void split_pair(float x0, float x1, uint32_t (&w)[NP]) {
 #pragma unroll

@@ -153,7 +153,8 @@ __device__ __forceinline__ void row_strided(T (&acc)[ROWS], const V *const (&aro
                                             size_t first, size_t nvec) {
     for (; first + 31 + 3 * STRIDE < nvec; first += 4 * STRIDE, c += 4 * STRIDE) row_group<4, STRIDE>(acc, arow, x, c);
     if (first >= nvec) return;
-    // the same small number twice: which form stays within 48 registers depends on the caller
+    // the same small number twice: by warps the 64-bit form compiles to 48 registers,
+    // by CTAs the 32-bit form (a difference of at most 4 * STRIDE, exact modulo 2^32)
     const int rem = STRIDE == 32 ? (int)((int64_t)nvec - (int64_t)c) : (int)nvec - (int)c;
     const int left = (int)(nvec - first);  // at most 4 * STRIDE
     if (left > 3 * STRIDE) row_last<4, STRIDE>(acc, arow, x, c, rem);
@@ -191,7 +192,7 @@ __device__ __forceinline__ void row_serial(T (&acc)[ROWS], const V *const (&arow
 
 // FEW: few warps per SM, so the tail of a row loads at once (row_tail); with
 // many its extra loads cost more (32768 x 1023: 29 us, 33 with row_tail; 1024^2
-// the other way round).
+// the other way round).  Doubles are bound to 48 registers, five CTAs per SM.
 template <typename T, int VW, int ROWS, int UNROLL, bool FEW>
 __global__ void __launch_bounds__(kGemvThreads, VW == 2 ? 5 : 0)
     gemv_rows_kernel(GemvArgs a) {
@@ -204,7 +205,6 @@ __global__ void __launch_bounds__(kGemvThreads, VW == 2 ? 5 : 0)
     const V *x = reinterpret_cast<const V *>(static_cast<const T *>(a.x) + p * a.stride_x);
     T *y = static_cast<T *>(a.y) + p * a.stride_y;
     const size_t nvec = a.N / VW;
-    const size_t ldv = a.lda / VW;
     const T alpha = (T)a.alpha, beta = (T)a.beta;
 
     for (size_t row0 = warp * ROWS; row0 < a.M; row0 += nwarps * ROWS) {
@@ -216,7 +216,6 @@ __global__ void __launch_bounds__(kGemvThreads, VW == 2 ? 5 : 0)
             const size_t row = (row0 + r < a.M) ? row0 + r : a.M - 1;  // clamp; result discarded
             arow[r] = reinterpret_cast<const V *>(A + row * a.lda);
         }
-        (void)ldv;
         if constexpr (FEW) {
             size_t c = lane;
             for (; c + (UNROLL - 1) * 32 < nvec; c += UNROLL * 32) row_group<UNROLL, 32>(acc, arow, x, c);
@@ -243,17 +242,16 @@ __global__ void __launch_bounds__(kGemvThreads, VW == 2 ? 5 : 0)
     }
 }
 
-// Five CTAs per SM need 48 registers a thread (56: 16384^2 floats 166 -> 170 us,
-// 30000 x 4400 90 -> 95).  Rows of one group and a short rest pay 3 % for the
-// clamped last group (30000 x 4400 87 -> 90, one element at a time), rows that end
-// in three or four vectors gain up to 40 %.
-//
 // Long rows: a CTA owns RB rows at a time and all 256 threads stride across
 // each of them in 16-byte vectors (UNROLL per row in flight, x reused from
 // registers across the RB rows); the per-thread chains are combined by a
 // fixed butterfly per warp and a fixed-order sum over the 8 warps in shared
 // memory.  The units are 8 times smaller than a warp's rows, so a 16384^2
 // product is thousands of CTAs and the last partial wave costs little.
+// SERIAL: the rest of a row one vector at a time (row_serial), else as one group
+// (row_strided).  Both compile to 48 registers with 16-byte vectors, which is five
+// CTAs per SM, without a bound that says so (at 56 16384^2 floats took 170 us, 166
+// at 48); bounds on the float kernels spilled.
 template <typename T, int VW, int RB, int UNROLL, bool SERIAL>
 __global__ void __launch_bounds__(kGemvThreads)
     gemv_rowblock_kernel(GemvArgs a) {
