@@ -65,3 +65,18 @@ def test_small_products_run_on_single_ctas(cuda, M, N, K):
     assert len(names) == 3 and "Li3ELb0E" in names[2]
     g.matmul(A, B, M, N, K, C=C, trans_b=True, engine="tc_fp8")
     assert bool((C == K).all())
+
+
+# row blocks of 512 (the last partial): single CTAs, or blocks wide enough for either
+@pytest.mark.parametrize("M,N,K", [(2300, 700, 1500), (1100, 19200, 1030)])
+def test_host_pipeline_on_varied_scales(cuda, M, N, K):
+    """Each row block contracts with its own part of the plan."""
+    import torch
+    rng = np.random.default_rng(M)
+    A, B = (torch.from_numpy(np.ascontiguousarray(_operand(rng, r, K, "all")).ravel()) for r in (M, N))
+    want = g.matmul(A.to(cuda), B.to(cuda), M, N, K, trans_b=True, engine="tc_fp8").cpu()
+    C = torch.full((M * N,), float("nan")).pin_memory()
+    g.matmul_host(A.pin_memory(), B.pin_memory(), M, N, K, C, trans_b=True, engine="tc_fp8")
+    torch.cuda.synchronize()
+    assert g.device_faults() == 0
+    assert torch.equal(C, want)
