@@ -534,21 +534,30 @@ Source source(const float *p, int64_t ld, int64_t rows, int64_t stride, int64_t 
 
 }  // namespace direct
 
+// Microseconds of either way in each mode: launches and set-up, a wave of tiles
+// beyond the first (two-pass: any wave), 64 k of a tile (64-row tiles of width 32,
+// 128-row tiles of width 32 and of 64; two-pass 128 or, on pairs, 256 x 256), a MB
+// of C by plain stores; the share that 64 k take longer where A or B is read in
+// pairs or stored across k; the split pass in TB/s along and across k.  Least
+// squares of the logarithms over 1500 random products (device time, B200); four
+// in five of 900 others lie within 20 %.
+struct Costs {
+    double start, wave, slice[3], c_mb, a_pairs, a_across, b_pairs, b_across;
+    double two_start, two_wave, two_slice, two_c_mb, split_along, split_across;
+};
+static const Costs kCosts[3] = {
+    {6.5, 1.8, {0.32, 0.60, 0.73}, 0.73, 0.47, 0.28, 0.22, 0.11, 11.8, 2.4, 0.36, 0.39, 5.5, 4.8},
+    {7.15, 2.3, {0.44, 0.71, 0.91}, 0.71, 0.49, 0.27, 0.18, 0.06, 15.0, 1.2, 0.90, 0.38, 6.3, 5.1},
+    {7.1, 2.2, {0.64, 0.96, 1.27}, 0.76, 0.28, 0.14, 0.16, 0.09, 14.3, 0.7, 1.93, 0.36, 5.9, 5.1}};
+
 // Tile width of the one-launch contraction for a product, 0 where the
-// two-pass path serves it: whichever of the two is estimated faster.
-//
-// Microseconds per 64 k of one tile, and per launch, from a sweep of 36 shapes
-// (device time, B200).  A 64-row tile of width 32, a 128-row tile of width 32
-// and of width 64 take 0.40 / 0.62 / 0.87 (BF16), 0.52 / 0.72 / 1.07 (split3)
-// and 0.75 / 1.05 / 1.42 (split6), about twice that where an operand has to be
-// read in pairs, and 5 per further wave of tiles; the two-pass contraction
-// 0.30 / 0.85 / 1.85 on its wider tiles, after a split pass at 6.3 TB/s (5.0 where
-// an operand is stored across k) and two more launches.  Either side of the
-// line, direct against two-pass: 64 x 4096 x 8192 BF16 56 and 86 us, split3 69 and
-// 200, split6 100 and 351; 1024^3 split3 21 and 27, BF16 18 and 16; 512^3 BF16 9.5
-// and 12.8; 1000 x 777 x 1100 BF16 18 and 22; 1536^3 split3 54 and 37; 128 x 128 x
-// 4096 BF16 39 and 28; 64 x 4095 x 8191 BF16 (pairs) 127 and 103; 2000 x 2000 x 100
-// BF16 24 and 13; seven of 16 x 3688 x 3320 BF16 183 and 133.
+// two-pass path serves it: whichever of the two is estimated faster, the one
+// launch by 8 % at least.  Over the 2400 products that loses 0.6 % against the
+// better of the two each time.  Either side of the line, direct against two-pass:
+// 64 x 4096 x 8192 BF16 56 and 86 us, split3 69 and 200, split6 100 and 351; 1024^3
+// split3 21 and 27, BF16 18 and 16; 512^3 BF16 9.5 and 12.8; 1000 x 777 x 1100 BF16 18
+// and 22; 1536^3 split3 54 and 37; 2000 x 2000 x 100 BF16 24 and 13; seven of 16 x 3688
+// x 3320 BF16 183 and 133, of 31 x 1782 x 1419 split6 71 and 111.
 int direct_width(const gatlas_matmul_desc *d, const Geometry &g, const float *A, const float *B, const float *C) {
     using namespace direct;
     if (d->engine == GATLAS_ENGINE_TC_FP8) return 0;  // block scales need whole 128 x 128 blocks first
@@ -558,28 +567,31 @@ int direct_width(const gatlas_matmul_desc *d, const Geometry &g, const float *A,
     // K beyond the transposing split's grid stays refused there
     if ((g.ta || !g.tb) && g.K > 65535 * 64) return 0;
     const int mode = d->engine == GATLAS_ENGINE_TC_BF16 ? 0 : d->engine == GATLAS_ENGINE_TC_SPLIT3 ? 1 : 2;
-    static const double kDirect[3][3] = {{0.40, 0.62, 0.87}, {0.52, 0.72, 1.07}, {0.75, 1.05, 1.42}};
-    static const double kPairs[3] = {2.2, 1.9, 1.45}, kTwoPass[3] = {0.30, 0.85, 1.85};
-    const double sms = sm_count(), slices = (double)((g.K + kSlice - 1) / kSlice);
-    auto waves = [](double tiles, double units) { return std::ceil(tiles / units); };
-    auto tiles = [&](int64_t m, int64_t n) { return (double)((g.M + m - 1) / m) * (double)((g.N + n - 1) / n) * (double)g.batch; };
-    const bool pairs = source(A, g.lda, g.M, g.stride_a, g.batch, g.ta).kind == kAlong ||
-                       source(B, g.ldb, g.N, g.stride_b, g.batch, !g.tb).kind == kAlong;
-    auto direct_us = [&](int bn) {
-        const double per_slice = kDirect[mode][g.M <= 64 ? 0 : bn == 32 ? 1 : 2] * (pairs ? kPairs[mode] : 1.0);
-        const double w = waves(tiles(128, bn), sms);
-        return 4.0 + w * slices * per_slice + (w - 1) * 5.0;
+    const Costs &c = kCosts[mode];
+    const double sms = sm_count(), slices = (double)((g.K + kSlice - 1) / kSlice), batch = (double)g.batch;
+    const auto waves = [&](int64_t m, int64_t n, double units) {
+        return std::ceil((double)((g.M + m - 1) / m) * (double)((g.N + n - 1) / n) * batch / units);
+    };
+    const int ka = source(A, g.lda, g.M, g.stride_a, g.batch, g.ta).kind;
+    const int kb = source(B, g.ldb, g.N, g.stride_b, g.batch, !g.tb).kind;
+    const bool reads_c = d->gemm && d->beta != 0.0;
+    const double c_mb = batch * (double)g.M * (double)g.N * 4e-6 * (reads_c ? 2 : 1);
+    const double slower = 1.0 + (ka == kAlong ? c.a_pairs : ka == kAcross ? c.a_across : 0.0) +
+                          (kb == kAlong ? c.b_pairs : kb == kAcross ? c.b_across : 0.0);
+    const auto direct_us = [&](int bn) {
+        const double w = waves(128, bn, sms);
+        return c.start + w * slices * c.slice[g.M <= 64 ? 0 : bn == 32 ? 1 : 2] * slower + (w - 1) * c.wave + c_mb * c.c_mb;
     };
     const bool pair = mode != 0 && g.M > BM;
-    const double k_bytes = (double)g.batch * (double)g.K * (4 + 2 * (mode + 1));
-    const double split_us = k_bytes * ((double)g.M / (g.ta ? 5.0e6 : 6.3e6) + (double)g.N / (g.tb ? 6.3e6 : 5.0e6));
-    // C by plain stores (beta, or rows not 16-byte aligned): 1 us per MB
-    const bool plain_c = (d->gemm && d->beta != 0.0) || g.ldc % 4 != 0 || !aligned16(C) || (g.batch > 1 && g.stride_c % 4 != 0);
-    const double two_pass_us = 9.0 + split_us +
-                               waves(tiles(pair ? 256 : 128, 256), pair ? sms / 2 : sms) * slices * kTwoPass[mode] +
-                               (plain_c ? (double)g.batch * (double)g.M * (double)g.N * 4 * 1e-6 : 0.0);
+    const bool plain_c = reads_c || g.ldc % 4 != 0 || !aligned16(C) || (g.batch > 1 && g.stride_c % 4 != 0);
+    const double w2 = waves(pair ? 256 : 128, 256, pair ? sms / 2 : sms);
+    const double mb_per_row = batch * (double)g.K * (4 + 2 * (mode + 1)) * 1e-6;
+    const double split_us = mb_per_row * ((double)g.M / (g.ta ? c.split_across : c.split_along) +
+                                          (double)g.N / (g.tb ? c.split_along : c.split_across));
+    const double two_pass_us =
+        c.two_start + split_us + w2 * (slices * c.two_slice + c.two_wave) + (plain_c ? c_mb * c.two_c_mb : 0.0);
     const double us32 = direct_us(32), us64 = g.M <= 64 ? us32 : direct_us(64);
-    if (std::min(us32, us64) > two_pass_us) return 0;
+    if (std::min(us32, us64) * 1.08 > two_pass_us) return 0;
     return us32 <= us64 ? 32 : 64;
 }
 
